@@ -310,13 +310,29 @@ __global__ void __launch_bounds__(kKtThreads) k_kt_vec(int op, size_t n, TVector
         last = atomicAdd(red.counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
+    if (!last) return;
+    // the CTA sums, added by the whole last CTA: thread i takes partials i, i + 256, ... and
+    // a fixed tree adds the threads. (One thread adding all 2 x 296 of them kept the grid
+    // waiting on a chain of L2 round trips, four such steps an iteration: the gradient of 4 RK4
+    // steps on the 64 x 64 cavity, K = 5, took 189 ms with it and takes 150 ms without.)
     __threadfence();
-    double a = 0.0, b = 0.0;
-    for (unsigned k = 0; k < gridDim.x; ++k) {
-        a += __ldcg(&red.partials[k]);
-        b += __ldcg(&red.partials[gridDim.x + k]);
+    d0 = d1 = 0.0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
+        d0 += __ldcg(&red.partials[k]);
+        d1 += __ldcg(&red.partials[gridDim.x + k]);
     }
+    s0[threadIdx.x] = d0;
+    s1[threadIdx.x] = d1;
+    __syncthreads();
+    for (int h = kKtThreads / 2; h > 0; h >>= 1) {
+        if ((int)threadIdx.x < h) {
+            s0[threadIdx.x] += s0[threadIdx.x + h];
+            s1[threadIdx.x] += s1[threadIdx.x + h];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x != 0) return;
+    const double a = s0[0], b = s1[0];
     *red.counter = 0u;
     kt_finish(op, a, b, sc, max_iter);
     if (op == KT_XR && has_handle) cudaGraphSetConditional(h, sc->done ? 0u : 1u);
