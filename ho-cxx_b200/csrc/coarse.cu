@@ -1,18 +1,23 @@
 // coarse.cu -- the coarse part of the two-level Poisson preconditioner (sm_100a).
 //
-// Level 0 of the coarse space holds one value per element (P0); its smoothed-aggregation
-// hierarchy is built on the host (host_amg.cpp) down to a level of at most kDenseMax
-// rows, whose inverse is precomputed. One V(1,1) cycle with SPAI-0 smoothing is linear
-// in f, so every other level's cycle is stored as three fixed row-padded operators,
+// Level 0 is the coarse space itself: one value per mesh vertex off the Dirichlet boundary,
+// interpolated bilinearly in each element (order 1: one value per element). Its
+// smoothed-aggregation hierarchy is built on the host (host_amg.cpp) down to a level of at
+// most kDenseMax rows, whose inverse is precomputed. One V(1,1) cycle with SPAI-0 smoothing
+// is linear in f, so every level's cycle is stored as three fixed row-padded operators,
 //   f_next = M f,   u = S f + Q u_next,
 // and a cycle is a chain of matrix-vector products with no intermediate residual or
 // correction vectors:
-//   downs    f_{l+1} = M_l f_l              l = 0 .. d-1   (k_coarse_rows)
-//   coarsest u_d = A_d^{-1} f_d                             (k_dense_gemv)
-//   ups      u_l = S_l f_l + Q_l u_{l+1}    l = d-1 .. 1   (k_coarse_rows)
-// The cycle ends with level 0's own up step u0 = S0 f0 + Q0 u1, one value per element,
-// which the fine smoothing kernel (krylov.cu, k_mf_post) reads for each element and its
-// four face neighbours.
+//   restriction  f_0[v] = the element moments that meet in v   (k_vertex_rhs)
+//   downs    f_{l+1} = M_l f_l              l = 0 .. d-1       (k_coarse_rows)
+//   coarsest u_d = A_d^{-1} f_d                                (k_dense_gemv)
+//   ups      u_l = S_l f_l + Q_l u_{l+1}    l = d-1 .. 0       (k_coarse_rows)
+// The combination (krylov.cu, k_post_b) reads u_0 at each element's four corners.
+//
+// The moments (element_moments in rows.cuh) are kept by the kernels that write the
+// residual vectors, so the cycle reads 4 values per element and runs beside the fine
+// smoothing on a second stream. What bounds it is latency: four to six dependent launches
+// over a few hundred KB to a few MB each, all L2-resident.
 //
 // Every kernel spans all SMs and sums in a fixed order (fixed lane-to-entry assignment
 // and xor-shuffle trees), so results are bitwise reproducible.
@@ -57,10 +62,10 @@ __device__ __forceinline__ void ell_accumulate(const DevEll<T>& A, const X& x, c
 }
 
 // grid-wide down (f_next = M f) or up (u = S f + Q u_next): G lanes per row, the group's
-// lanes combine their partial sums with an xor-shuffle tree. XA is a plain vector, or
-// (the level-0 restriction) the right-hand side formed from the element sums.
-template <typename T, typename XA>
-__global__ void __launch_bounds__(256) k_coarse_rows(DevEll<T> A, XA xa, DevEll<T> B, const T* __restrict__ xb,
+// lanes combine their partial sums with an xor-shuffle tree.
+template <typename T>
+__global__ void __launch_bounds__(256) k_coarse_rows(DevEll<T> A, const T* __restrict__ xa, DevEll<T> B,
+                                                      const T* __restrict__ xb,
                                                       int has_b, T* __restrict__ y, const KrylovScalars* sc) {
     const bool skip = sc->done;  // read early: the round trip overlaps the loads
     const int G = A.g;
@@ -214,40 +219,57 @@ void dense_gemv(const DevEll<T>& W, const T* f, T* u, const KrylovScalars* sc, c
     k_dense_gemv<T><<<gd, 32 * kGemvWarps, 0, s>>>(W, f, u, sc);
 }
 
-// u0 of element c into every block slot that reads it (Precond::u0dst)
+// the element moments that meet in level-0 unknown r, summed in the table's order
 template <typename T>
-__device__ __forceinline__ void scatter_u0(const int* __restrict__ u0dst, T* __restrict__ ue5, int c, T a) {
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const int d = u0dst[c * 5 + k];
-        if (d >= 0) ue5[d] = a;
+__device__ __forceinline__ T vertex_sum(const int* __restrict__ v2e, int vw, const F0<T>& m, int r) {
+    T acc = T(0);
+    for (int k = 0; k < vw; ++k) {
+        const int e = __ldg(v2e + (size_t)r * vw + k);
+        if (e >= 0) acc += m[e];
     }
+    return acc;
 }
 
-// u0 = W f0 when the P0 level itself is the dense one (small meshes): f0 is formed from
-// the element sums as it is read, one warp per row, scalar loads
+// f_0 from the element moments, one thread per unknown
 template <typename T>
-__global__ void __launch_bounds__(32 * kGemvWarps) k_dense_gemv_f0(DevEll<T> W, BicgVectors<T> v,
-                                                                    const int* __restrict__ u0dst,
-                                                                    T* __restrict__ ue5, const KrylovScalars* sc,
-                                                                    int mode) {
+__global__ void __launch_bounds__(256) k_vertex_rhs(int n, const int* __restrict__ v2e, int vw, BicgVectors<T> v,
+                                                     T* __restrict__ f, const KrylovScalars* sc, int mode) {
+    const bool skip = sc->done;  // read early: the round trip overlaps the loads
+    const F0<T> m = f0_of(v, sc, mode);
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    const T a = vertex_sum<T>(v2e, vw, m, r);
+    if (!skip) f[r] = a;
+}
+
+// u_0 = W f_0 when level 0 itself is the dense one (small meshes): every CTA forms f_0 in its
+// shared memory (n values of T), then one warp per row. One launch instead of two: at 225
+// unknowns the extra reads (a few KB per CTA, L2-resident) cost less than a launch.
+template <typename T>
+__global__ void __launch_bounds__(32 * kGemvWarps) k_dense_gemv_f0(DevEll<T> W, const int* __restrict__ v2e, int vw,
+                                                                    BicgVectors<T> v, T* __restrict__ u,
+                                                                    const KrylovScalars* sc, int mode) {
+    extern __shared__ __align__(16) unsigned char f0_dyn[];
+    T* f = reinterpret_cast<T*>(f0_dyn);
     const bool skip = sc->done;
-    const F0<T> f = f0_of(v, sc, mode);
+    const F0<T> m = f0_of(v, sc, mode);
+    for (int r = threadIdx.x; r < W.n; r += 32 * kGemvWarps) f[r] = vertex_sum<T>(v2e, vw, m, r);
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     const int row = blockIdx.x * kGemvWarps + (threadIdx.x >> 5);
     if (row >= W.n) return;
     const T* wr = W.val + (size_t)row * W.w;
     T acc = T(0);
+#pragma unroll 8
     for (int k = lane; k < W.n; k += 32) acc += __ldg(wr + k) * f[k];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane == 0 && !skip) scatter_u0(u0dst, ue5, row, acc);
+    if (lane == 0 && !skip) u[row] = acc;
 }
 
-// level-0 restriction with the right-hand side formed from the element sums
-template <typename T>
-__global__ void __launch_bounds__(256) k_coarse_rows_f0(DevEll<T> M, BicgVectors<T> v, T* __restrict__ y,
-                                                         const KrylovScalars* sc, int mode);
+// largest dense level 0 whose right-hand side every CTA forms for itself (the shared memory
+// a launch gets without asking)
+constexpr size_t kGemvF0Bytes = 48 * 1024;
 
 template <typename T>
 unsigned rows_grid(const DevEll<T>& A) {
@@ -257,122 +279,49 @@ unsigned rows_grid(const DevEll<T>& A) {
     return (unsigned)(blocks < 1 ? 1 : blocks);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_coarse_rows_f0(DevEll<T> M, BicgVectors<T> v, T* __restrict__ y,
-                                                         const KrylovScalars* sc, int mode) {
-    // the same row loop as k_coarse_rows, gathering f0 = a + cb b + cc c
-    const bool skip = sc->done;
-    const F0<T> xa = f0_of(v, sc, mode);
-    const int G = M.g;
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int group = gid / G, sub = gid % G, ngroups = (int)(gridDim.x * blockDim.x) / G;
-    const int iters = (M.n + ngroups - 1) / ngroups;
-    for (int it = 0; it < iters; it += kRowBatch) {
-        T acc[kRowBatch];
-        int row[kRowBatch];
-        bool ok[kRowBatch];
-#pragma unroll
-        for (int r = 0; r < kRowBatch; ++r) {
-            acc[r] = T(0);
-            row[r] = group + (it + r) * ngroups;
-            ok[r] = it + r < iters && row[r] < M.n;
-        }
-        ell_accumulate<T>(M, xa, row, ok, G, sub, acc);
-#pragma unroll
-        for (int r = 0; r < kRowBatch; ++r) {
-            T a = acc[r];
-            for (int off = G >> 1; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-            if (sub == 0 && ok[r] && !skip) y[row[r]] = a;
-        }
-    }
-}
-
-// level-0 up step u0 = S0 f0 + Q0 u1 with the right-hand side formed from the element sums;
-// each row's value goes to the block slots that read it (scatter_u0)
-template <typename T>
-__global__ void __launch_bounds__(256) k_coarse_up0(DevEll<T> S, DevEll<T> Q, BicgVectors<T> v,
-                                                     const T* __restrict__ u1, const int* __restrict__ u0dst,
-                                                     T* __restrict__ ue5, const KrylovScalars* sc, int mode) {
-    const bool skip = sc->done;
-    const F0<T> xa = f0_of(v, sc, mode);
-    const int G = S.g;
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int group = gid / G, sub = gid % G, ngroups = (int)(gridDim.x * blockDim.x) / G;
-    const int iters = (S.n + ngroups - 1) / ngroups;
-    for (int it = 0; it < iters; it += kRowBatch) {
-        T acc[kRowBatch];
-        int row[kRowBatch];
-        bool ok[kRowBatch];
-#pragma unroll
-        for (int r = 0; r < kRowBatch; ++r) {
-            acc[r] = T(0);
-            row[r] = group + (it + r) * ngroups;
-            ok[r] = it + r < iters && row[r] < S.n;
-        }
-        ell_accumulate<T>(S, xa, row, ok, G, sub, acc);
-        ell_accumulate<T>(Q, u1, row, ok, G, sub, acc);
-#pragma unroll
-        for (int r = 0; r < kRowBatch; ++r) {
-            T a = acc[r];
-            for (int off = G >> 1; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-            if (sub == 0 && ok[r] && !skip) scatter_u0(u0dst, ue5, row[r], a);
-        }
-    }
-}
-
 }  // namespace
+
+// downs, coarsest solve and ups from level 0's right-hand side f0
+template <typename T>
+static void cycle_from(const Precond<T>& pc, const T* f0, const KrylovScalars* sc, cudaStream_t s) {
+    const int d = pc.nlev - 1;
+    for (int l = 0; l < d; ++l) {
+        const CoarseLevel<T>& L = pc.lev[l];
+        k_coarse_rows<T><<<rows_grid(L.M), 256, 0, s>>>(L.M, l ? L.f : f0, DevEll<T>(), nullptr, 0, pc.lev[l + 1].f, sc);
+    }
+    dense_gemv<T>(pc.dense, d ? pc.lev[d].f : f0, pc.lev[d].u, sc, s);
+    for (int l = d - 1; l >= 0; --l) {
+        const CoarseLevel<T>& L = pc.lev[l];
+        k_coarse_rows<T><<<rows_grid(L.S), 256, 0, s>>>(L.S, l ? L.f : f0, L.Q, pc.lev[l + 1].u, 1, L.u, sc);
+    }
+}
+
+template <typename T>
+static bool gemv_forms_f0(const Precond<T>& pc) {
+    return pc.nlev == 1 && (size_t)pc.dense.n * sizeof(T) <= kGemvF0Bytes;
+}
 
 template <typename T>
 cudaError_t coarse_cycle(const Precond<T>& pc, const BicgVectors<T>& v, const KrylovScalars* sc, int mode,
                          cudaStream_t s) {
-    const int d = pc.nlev - 1;
-    const unsigned gd = (unsigned)((pc.dense.n + kGemvWarps - 1) / kGemvWarps);
-    if (d == 0) {
-        k_dense_gemv_f0<T><<<gd, 32 * kGemvWarps, 0, s>>>(pc.dense, v, pc.u0dst, pc.ue5, sc, mode);
+    if (gemv_forms_f0(pc)) {
+        const unsigned gd = (unsigned)((pc.dense.n + kGemvWarps - 1) / kGemvWarps);
+        k_dense_gemv_f0<T><<<gd, 32 * kGemvWarps, pc.dense.n * sizeof(T), s>>>(pc.dense, pc.v2e, pc.vw, v, pc.lev[0].u, sc,
+                                                                               mode);
         return cudaGetLastError();
     }
-    k_coarse_rows_f0<T><<<rows_grid(pc.lev[0].M), 256, 0, s>>>(pc.lev[0].M, v, pc.lev[1].f, sc, mode);
-    for (int l = 1; l < d; ++l) {
-        const CoarseLevel<T>& L = pc.lev[l];
-        k_coarse_rows<T, const T*><<<rows_grid(L.M), 256, 0, s>>>(L.M, L.f, DevEll<T>(), nullptr, 0,
-                                                                   pc.lev[l + 1].f, sc);
-    }
-    dense_gemv<T>(pc.dense, pc.lev[d].f, pc.lev[d].u, sc, s);
-    for (int l = d - 1; l >= 1; --l) {
-        const CoarseLevel<T>& L = pc.lev[l];
-        k_coarse_rows<T, const T*><<<rows_grid(L.S), 256, 0, s>>>(L.S, L.f, L.Q, pc.lev[l + 1].u, 1, L.u, sc);
-    }
-    const CoarseLevel<T>& L0 = pc.lev[0];
-    k_coarse_up0<T><<<rows_grid(L0.S), 256, 0, s>>>(L0.S, L0.Q, v, pc.lev[1].u, pc.u0dst, pc.ue5, sc, mode);
+    const int n0 = pc.lev[0].n;
+    k_vertex_rhs<T><<<(unsigned)((n0 + 255) / 256), 256, 0, s>>>(n0, pc.v2e, pc.vw, v, pc.lev[0].f, sc, mode);
+    cycle_from<T>(pc, pc.lev[0].f, sc, s);
     return cudaGetLastError();
 }
 
-// The whole cycle on a plain level-0 right-hand side f0 (N entries, zero-padded to a
-// multiple of 4): u0 = cycle(f0) in pc.lev[0].u, level 0's own up step included. Used by
-// the transposed solve of the adjoint, whose preconditioner forms f0 in its own kernel.
+// The whole cycle on a plain level-0 right-hand side f0 (zero-padded to a multiple of 4):
+// u0 = cycle(f0) in pc.lev[0].u. Used by the transposed solve of the adjoint, whose
+// preconditioner forms f0 in its own kernel.
 template <typename T>
 cudaError_t coarse_cycle_vec(const Precond<T>& pc, const T* f0, const KrylovScalars* sc, cudaStream_t s) {
-    const int d = pc.nlev - 1;
-    if (d < 0) return cudaSuccess;
-    const unsigned gd = (unsigned)((pc.dense.n + kGemvWarps - 1) / kGemvWarps);
-    if (d == 0) {
-        dense_gemv<T>(pc.dense, f0, pc.lev[0].u, sc, s);
-        return cudaGetLastError();
-    }
-    k_coarse_rows<T, const T*><<<rows_grid(pc.lev[0].M), 256, 0, s>>>(pc.lev[0].M, f0, DevEll<T>(), nullptr, 0,
-                                                                       pc.lev[1].f, sc);
-    for (int l = 1; l < d; ++l) {
-        const CoarseLevel<T>& L = pc.lev[l];
-        k_coarse_rows<T, const T*><<<rows_grid(L.M), 256, 0, s>>>(L.M, L.f, DevEll<T>(), nullptr, 0,
-                                                                   pc.lev[l + 1].f, sc);
-    }
-    dense_gemv<T>(pc.dense, pc.lev[d].f, pc.lev[d].u, sc, s);
-    for (int l = d - 1; l >= 1; --l) {
-        const CoarseLevel<T>& L = pc.lev[l];
-        k_coarse_rows<T, const T*><<<rows_grid(L.S), 256, 0, s>>>(L.S, L.f, L.Q, pc.lev[l + 1].u, 1, L.u, sc);
-    }
-    const CoarseLevel<T>& L0 = pc.lev[0];
-    k_coarse_rows<T, const T*><<<rows_grid(L0.S), 256, 0, s>>>(L0.S, f0, L0.Q, pc.lev[1].u, 1, L0.u, sc);
+    if (pc.nlev > 0) cycle_from<T>(pc, f0, sc, s);
     return cudaGetLastError();
 }
 
@@ -386,35 +335,27 @@ int coarse_vec_launches(const Precond<T>& pc) {
 template <typename T>
 int coarse_launches(const Precond<T>& pc) {
     if (pc.nlev <= 0) return 0;
-    const int d = pc.nlev - 1;
-    return d == 0 ? 1 : d + 1 + (d - 1) + 1;
+    return gemv_forms_f0(pc) ? 1 : 2 * pc.nlev;
 }
 
-// Algorithmic bytes of one coarse cycle as coarse_cycle launches it: every row-padded
-// operator's values and column indices, the dense inverse, each level's right-hand side
-// read and result written; the level-0 right-hand side is formed from three element-sum
-// vectors.
+// Algorithmic bytes of one coarse cycle as coarse_cycle launches it: the element moments (p's
+// and s's are combinations of up to three vectors) and the restriction table, every
+// row-padded operator's values and column indices, the dense inverse, each level's
+// right-hand side read and result written.
 template <typename T>
-int coarse_cycle_bytes(const Precond<T>& pc) {
-    if (pc.nlev <= 0) return 0;
+double coarse_cycle_bytes(const Precond<T>& pc) {
+    if (pc.nlev <= 0) return 0.0;
     const int d = pc.nlev - 1;
     auto ell = [](const DevEll<T>& A) { return (double)A.n * A.w * (sizeof(T) + (A.col ? 4 : 0)); };
     const double dsz = pc.dense.val16 ? 2.0 : (double)sizeof(T);
-    double b = (double)pc.dense.n * pc.dense.w * dsz + 2.0 * pc.dense.n * sizeof(T);
-    if (d == 0) return (int)(b + 3.0 * pc.dense.n * sizeof(T));
-    b += ell(pc.lev[0].M) + 3.0 * pc.lev[0].n * sizeof(T) + pc.lev[1].n * sizeof(T);
-    for (int l = 1; l < d; ++l) b += ell(pc.lev[l].M) + (double)(pc.lev[l].n + pc.lev[l + 1].n) * sizeof(T);
-    for (int l = d - 1; l >= 1; --l)
+    const int n0 = pc.lev[0].n;
+    double b = (double)n0 * pc.vw * (4.0 + 3.0 * sizeof(T)) + (double)n0 * sizeof(T);
+    b += (double)pc.dense.n * pc.dense.w * dsz + 2.0 * pc.dense.n * sizeof(T);
+    for (int l = 0; l < d; ++l) {
+        b += ell(pc.lev[l].M) + (double)(pc.lev[l].n + pc.lev[l + 1].n) * sizeof(T);
         b += ell(pc.lev[l].S) + ell(pc.lev[l].Q) + (double)(2 * pc.lev[l].n + pc.lev[l + 1].n) * sizeof(T);
-    b += ell(pc.lev[0].S) + ell(pc.lev[0].Q) + (double)(4 * pc.lev[0].n + pc.lev[1].n) * sizeof(T);
-    return (int)b;
-}
-
-template <typename T>
-CoarseOut<T> coarse_out(const Precond<T>& pc) {
-    CoarseOut<T> c;
-    c.ue5 = pc.ue5;
-    return c;
+    }
+    return b;
 }
 
 #define HO2D_INSTANTIATE_COARSE(T)                                                                   \
@@ -423,8 +364,7 @@ CoarseOut<T> coarse_out(const Precond<T>& pc) {
     template int coarse_launches<T>(const Precond<T>&);                                              \
     template cudaError_t coarse_cycle_vec<T>(const Precond<T>&, const T*, const KrylovScalars*, cudaStream_t); \
     template int coarse_vec_launches<T>(const Precond<T>&);                                          \
-    template CoarseOut<T> coarse_out<T>(const Precond<T>&);                                          \
-    template int coarse_cycle_bytes<T>(const Precond<T>&);
+    template double coarse_cycle_bytes<T>(const Precond<T>&);
 
 HO2D_INSTANTIATE_COARSE(double)
 HO2D_INSTANTIATE_COARSE(float)

@@ -92,6 +92,10 @@ struct KrylovScalars {
     int stalled, pad2;
 };
 
+// Whether a finished FP32 solve reduced its residual at all (false for NaN): BiCGSTAB can break
+// down in FP32, and its x may then hold anything.
+__host__ __device__ inline bool krylov_usable(const KrylovScalars& sc) { return sc.rnorm2 <= sc.bnorm2; }
+
 // A preconditioner application is skipped once the solve is done, and the second one of
 // an iteration (mode 1) also when the iteration exits early after its s update.
 __device__ __forceinline__ bool pc_skip(const KrylovScalars* sc, int mode) {

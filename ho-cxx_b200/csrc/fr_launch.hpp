@@ -108,11 +108,17 @@ struct PoisGeom {
 };
 
 // Matrix-free FR Laplacian (the Poisson operator) plus the preconditioner's element data.
-// Weight of the preconditioner's block smoothing step, z = e + w M (f - A e). Under-relaxing
-// the exact (or fitted) block inverse pays: on the 256 x 512 cylinder O-grid at K = 6 the
-// inner iterations per step fell by 18% (mixed) and 14% (FP64) from w = 1 to 0.7, and on
-// the backward-facing step by 5%.
-constexpr double kSmoothingWeight = 0.7;
+// Weight of the preconditioner's block smoothing step, z = P u0 + w M f.
+constexpr double kSmoothingWeight = 0.8;
+
+// The 1-D hat functions of the coarse space, [i*2+lr] at solution point i (lr = 0: 1 at
+// xi = -1, lr = 1: 1 at xi = +1): hp as the coarse function is interpolated to the points,
+// hr as a residual is tested with it. Forward operator: hr = hp times the quadrature weight;
+// transposed operator: the two exchanged.
+template <typename T>
+struct HatBases {
+    T hp[16], hr[16];
+};
 
 template <typename T>
 struct MfOp {
@@ -120,8 +126,7 @@ struct MfOp {
     PoisGeom<T> g;
     DevBases<T> b;
     const T* dinv;          // [N][K2][K2] inverse diagonal blocks, transposed ([rs][ij])
-    const T* rowsum;        // [N][5][K2] row sums of the 5 blocks of each element row
-    const int* bcol;        // [N][5] element of each block (slot 0 = self, 1 + ijp = neighbours)
+    HatBases<T> h;
     // optional BF16 copy of dinv (bit patterns), read by the FP32 smoother when present
     const unsigned short* dinv_bf16 = nullptr;
     // optional Kronecker-sum smoother (FP32): factors [N][4K^2 + 2K], the compact index of
@@ -129,8 +134,6 @@ struct MfOp {
     const T* kron_f = nullptr;
     const int* kron_x = nullptr;
     const T* kron_exact = nullptr;
-    // [N][5][K2] the smoother's element inverse applied to each block row sum (k_make_w)
-    const T* W = nullptr;
     // FP32 operator kernels stage their inputs in shared memory by bulk copies
     // (apply_stage.cuh) instead of reading them through L2 prefetches
     int staged = 0;
@@ -146,15 +149,15 @@ struct BicgVectors {
     const T* b;
     T *tv, *tg;    // incoming face traces of the operand of the next operator application
     T *xtv, *xtg;  // incoming face traces of x (initial residual)
-    // element sums (N entries, zero-padded) of r, of v, and of p in two buffers that
-    // alternate with the iteration count: the coarse right-hand sides P^T p and P^T s are
-    // linear combinations of them, formed wherever they are read
+    // element moments [N][4] (the element's values tested with its four hats, element_moments)
+    // of r, of v, and of p in two buffers that alternate with the iteration count: those of p
+    // and s are linear combinations of them, formed where they are read
     T *er, *ev, *ep[2];
     T* zf;  // the fine part M f of the current preconditioner application (k_post_a)
 };
 
-// The level-0 coarse right-hand side of one preconditioner application, formed where it
-// is read: f0[e] = a[e] + cb b[e] + cc c[e].
+// The element moments of one preconditioner application's operand, formed where they are
+// read: f0[e] = a[e] + cb b[e] + cc c[e], e = 4 el + corner.
 //   mode 0 (p = r + beta (p - omega v)):  f0 = er + beta ep_prev - beta omega ev
 //                                          (= er on the first iteration)
 //   mode 1 (s = r - alpha v):             f0 = er - alpha ev
@@ -203,7 +206,7 @@ struct DevEll {
     const unsigned short* val16 = nullptr;
 };
 
-// One level of the coarse hierarchy (level 0 = one value per element). Its V(1,1) cycle
+// One level of the coarse hierarchy (level 0: the coarse space's own values). Its V(1,1) cycle
 // is f_next = M f and u = S f + Q u_next (host_amg.hpp has the formulas).
 template <typename T>
 struct CoarseLevel {
@@ -222,22 +225,15 @@ struct Precond {
     double omega = 1.0;  // weight of the block-Jacobi smoothing step
     CoarseLevel<T> lev[kMaxLevels];
     DevEll<T> dense;  // row-major inverse of the coarsest operator (col == nullptr)
-    // level-0 result delivered per element: ue5[5 el + s] = u0 of the element in block slot s
-    // of element el (s = 0 itself, 1 + ijp its face neighbours; 0 where there is none);
-    // u0dst[5 c + k] lists the slots element c's value goes to (-1: unused)
-    T* ue5 = nullptr;
-    const int* u0dst = nullptr;
+    // the coarse space: conn[4 el + c] = level-0 unknown at corner c of element el (-1: none),
+    // v2e[vw v + k] = the element moments (4 el + c) that meet in unknown v (-1: unused)
+    const int* conn = nullptr;
+    const int* v2e = nullptr;
+    int vw = 0;
 };
 
-// What the fine smoothing step needs of the coarse result: u0 at each element's five block
-// slots (the whole cycle, level 0's up step included, ran before it).
-template <typename T>
-struct CoarseOut {
-    const T* ue5 = nullptr;  // [N][5]: u0 of each element's five block slots (Precond::ue5)
-};
-
-// enqueues the coarse part of one preconditioner application (mode 0: on P^T p, mode 1:
-// on P^T s, both formed from the element sums in v)
+// enqueues the coarse part of one preconditioner application (mode 0: on p, mode 1: on s,
+// restricted from the element moments in v); the result is pc.lev[0].u
 template <typename T>
 cudaError_t coarse_cycle(const Precond<T>& pc, const BicgVectors<T>& v, const KrylovScalars* sc, int mode,
                          cudaStream_t s);
@@ -249,9 +245,7 @@ cudaError_t coarse_cycle_vec(const Precond<T>& pc, const T* f0, const KrylovScal
 template <typename T>
 int coarse_vec_launches(const Precond<T>& pc);
 template <typename T>
-CoarseOut<T> coarse_out(const Precond<T>& pc);
-template <typename T>
-int coarse_cycle_bytes(const Precond<T>& pc);
+double coarse_cycle_bytes(const Precond<T>& pc);
 
 template <typename T>
 cudaError_t krylov_init(const MfOp<T>& op, const BicgVectors<T>& v, const ReduceScratch& rs, cudaStream_t s);
@@ -301,10 +295,6 @@ cudaError_t rows_to_f32(const double* src, long long ss, const int* idx, float* 
 cudaError_t rows_to_bf16(const double* src, long long ss, unsigned short* dst, long long ds, int rows, int cols,
                          cudaStream_t s);
 cudaError_t dense_invert_device(double* a, int n, int w, cudaStream_t s, bool* singular);
-// W = M rowsum for the 5 block slots of every element ([N][5][K2], T), with the smoother
-// op selects (its element inverse M: exact blocks, BF16 blocks or Kronecker-sum factors)
-template <typename T>
-cudaError_t krylov_make_w(const MfOp<T>& op, T* W, KrylovScalars* sc, cudaStream_t s);
 
 // out[0..1] = FP64 force on a body from its boundary points' precomputed coefficients
 // (forces.cu): coef [npts][4], idx = index of each point in the boundary arrays

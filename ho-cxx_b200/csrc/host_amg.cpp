@@ -2,8 +2,8 @@
 //
 // The device preconditioner is two-level: damped element block-Jacobi on the FR operator
 // (exact solves of each element's K^2 x K^2 diagonal block) plus a correction in the
-// space of element-wise constants (P0). The P0 Galerkin operator A1 = P^T A P has one
-// row per element and the element adjacency as its pattern (5 entries per row); it is
+// space of continuous bilinear functions on the mesh vertices (CoarseSpace). Its operator has
+// one row per free vertex and 9 entries per row on a structured patch; it is
 // solved approximately by one V-cycle of smoothed-aggregation AMG -- the coarsening
 // family of the reference's AMGCL setup (src/HO_2D.hpp:54, src/HO_2D.cpp:3066-3072),
 // written here from the published method (Vanek, Mandel & Brezina 1996):
@@ -293,6 +293,109 @@ Ell to_ell(const Csr& A) {
             E.val[(size_t)i * E.w + (k - A.ptr[i])] = A.val[k];
         }
     return E;
+}
+
+CoarseSpace coarse_space(const Mesh& m, const Bases& B, const BoundaryConditions& bc) {
+    const int N = m.n_el, K = B.K, lin = m.lnod - 1;
+    CoarseSpace s;
+    s.hp.assign((size_t)K * 2, 1.0);
+    s.hr.assign((size_t)K * 2, 1.0);
+    s.conn.assign((size_t)N * 4, -1);
+    if (K == 1) {
+        s.n = N;
+        s.vw = 1;
+        s.hp[1] = s.hr[1] = 0.0;
+        s.v2e.resize(N);
+        for (int el = 0; el < N; ++el) {
+            s.conn[(size_t)el * 4] = el;
+            s.v2e[el] = el * 4;
+        }
+        return s;
+    }
+    for (int i = 0; i < K; ++i)
+        for (int lr = 0; lr < 2; ++lr) {
+            s.hp[i * 2 + lr] = 0.5 * (lr ? 1.0 + B.xs[i] : 1.0 - B.xs[i]);
+            s.hr[i * 2 + lr] = 0.5 * K * B.w[i] * s.hp[i * 2 + lr];
+        }
+    const int corner[4] = {tensor2fem(0, 0, lin), tensor2fem(lin, 0, lin), tensor2fem(lin, lin, lin),
+                           tensor2fem(0, lin, lin)};
+    std::vector<int> id(m.node_xy.size() / 2, -1);  // -2: on a Dirichlet edge
+    for (int e = 0; e < m.n_eb; ++e) {
+        if (bc.sw_p[e] != 0) continue;
+        for (int q = 0; q < 2; ++q) id[m.elem_nodes[m.be_el[e]][corner[(m.be_side[e] + q) % 4]]] = -2;
+    }
+    std::vector<int> cnt;
+    for (int el = 0; el < N; ++el)
+        for (int c = 0; c < 4; ++c) {
+            int& v = id[m.elem_nodes[el][corner[c]]];
+            if (v == -2) continue;
+            if (v == -1) {
+                v = s.n++;
+                cnt.push_back(0);
+            }
+            s.conn[(size_t)el * 4 + c] = v;
+            s.vw = std::max(s.vw, ++cnt[v]);
+        }
+    s.v2e.assign((size_t)s.n * s.vw, -1);
+    std::fill(cnt.begin(), cnt.end(), 0);
+    for (int q = 0; q < N * 4; ++q)
+        if (s.conn[q] >= 0) s.v2e[(size_t)s.conn[q] * s.vw + cnt[s.conn[q]]++] = q;
+    return s;
+}
+
+Csr coarse_operator(const CoarseSpace& s, const Bases& B, const std::vector<double>* g) {
+    const int K = B.K, K2 = K * K, N = (int)(s.conn.size() / 4);
+    // corner c = (x, y) end: its hat is h_x(xi) h_y(eta), its xi derivative +-1/2 h_y
+    const int cx[4] = {0, 1, 1, 0}, cy[4] = {0, 0, 1, 1};
+    std::vector<double> Ae((size_t)N * 16);
+#pragma omp parallel for schedule(static)
+    for (int el = 0; el < N; ++el) {
+        // sums over the points of w G11 h_y h_y', w G22 h_x h_x', w G12 h_y h_x'
+        double s11[2][2] = {}, s22[2][2] = {}, s12[2][2] = {};
+        for (int j = 0; j < K; ++j)
+            for (int i = 0; i < K; ++i) {
+                const size_t p = (size_t)el * K2 + j * K + i;
+                const double w = 0.25 * K2 * B.w[i] * B.w[j];
+                for (int a = 0; a < 2; ++a)
+                    for (int b = 0; b < 2; ++b) {
+                        s11[a][b] += w * g[0][p] * s.hp[j * 2 + a] * s.hp[j * 2 + b];
+                        s22[a][b] += w * g[2][p] * s.hp[i * 2 + a] * s.hp[i * 2 + b];
+                        s12[a][b] += w * g[1][p] * s.hp[j * 2 + a] * s.hp[i * 2 + b];
+                    }
+            }
+        for (int a = 0; a < 4; ++a)
+            for (int b = 0; b < 4; ++b) {
+                const double xa = cx[a] ? 0.5 : -0.5, ya = cy[a] ? 0.5 : -0.5;
+                const double xb = cx[b] ? 0.5 : -0.5, yb = cy[b] ? 0.5 : -0.5;
+                Ae[(size_t)el * 16 + a * 4 + b] = -(xa * xb * s11[cy[a]][cy[b]] + ya * yb * s22[cx[a]][cx[b]] +
+                                                    xa * yb * s12[cy[a]][cx[b]] + xb * ya * s12[cy[b]][cx[a]]);
+            }
+    }
+    Csr A;
+    A.n = A.m = s.n;
+    A.ptr.assign((size_t)s.n + 1, 0);
+    std::vector<std::pair<int, double>> row;
+    for (int v = 0; v < s.n; ++v) {
+        row.clear();
+        for (int k = 0; k < s.vw; ++k) {
+            const int q = s.v2e[(size_t)v * s.vw + k];
+            if (q < 0) continue;
+            for (int b = 0; b < 4; ++b) {
+                const int c = s.conn[(size_t)(q / 4) * 4 + b];
+                if (c >= 0) row.push_back({c, Ae[(size_t)(q / 4) * 16 + (q % 4) * 4 + b]});
+            }
+        }
+        std::stable_sort(row.begin(), row.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+        for (size_t k = 0; k < row.size(); ++k) {
+            if (k && row[k].first == row[k - 1].first) A.val.back() += row[k].second;
+            else {
+                A.col.push_back(row[k].first);
+                A.val.push_back(row[k].second);
+            }
+        }
+        A.ptr[(size_t)v + 1] = (int)A.col.size();
+    }
+    return A;
 }
 
 Csr p0_coarse_operator(const PoissonOperator& op, int N) {

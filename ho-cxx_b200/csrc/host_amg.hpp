@@ -1,4 +1,5 @@
-// host_amg.hpp -- P0 coarse operator and its smoothed-aggregation hierarchy (host setup).
+// host_amg.hpp -- coarse space of the Poisson preconditioner and its smoothed-aggregation
+// hierarchy (host setup).
 #pragma once
 
 #include <vector>
@@ -41,10 +42,31 @@ struct Ell {
 Ell to_ell(const Csr& A);
 
 struct CoarseHierarchy {
-    std::vector<AmgLevel> levels;  // levels[0] is the P0 (one value per element) operator
+    std::vector<AmgLevel> levels;  // levels[0] is the coarse space's own operator
     int n_dense = 0;
     std::vector<double> dense_inv;  // row-major inverse of the coarsest operator
 };
+
+// The coarse space: a value at every mesh vertex off the Dirichlet boundary, interpolated
+// bilinearly in each element's reference square. conn[4 el + c]: the unknown at corner c
+// ((-,-), (+,-), (+,+), (-,+)) or -1; v2e: per unknown the vw-wide list of the corners
+// (4 el + c, ascending; -1 pads) that meet in it; hp, hr [K][2]: the 1-D hats at the solution
+// points and the hats times K quadrature weights (HatBases, fr_launch.hpp). Unknowns are
+// numbered in the order the elements meet them, so they are as local as the elements.
+// At order 1 an element has one value and the space is the elements themselves (P = identity).
+struct CoarseSpace {
+    int n = 0, vw = 0;
+    std::vector<int> conn, v2e;
+    std::vector<double> hp, hr;
+};
+CoarseSpace coarse_space(const Mesh& m, const Bases& B, const BoundaryConditions& bc);
+// The bilinear finite-element Laplacian on that space, integrated with the solution points'
+// quadrature: -K^2 sum_q w_q grad phi_a . G grad phi_b over the contravariant coefficients
+// g[0..2] = G11, G12, G22 ([N][K][K]). On affine elements this is R A P of the FR operator to
+// rounding, because continuous functions have no jumps to lift; elsewhere it differs from it
+// by about 1% and is preferred for its 9-point rows (R A P has 21) and its symmetry, which
+// lets the transposed problem use the same hierarchy.
+Csr coarse_operator(const CoarseSpace& s, const Bases& B, const std::vector<double>* g);
 
 // A1 = P^T A P for P = element indicator: the sum of each K^2 x K^2 block.
 Csr p0_coarse_operator(const PoissonOperator& op, int N);

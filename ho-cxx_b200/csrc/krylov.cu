@@ -10,12 +10,17 @@
 // one operator application is one launch.
 //
 // Solver. Right-preconditioned BiCGSTAB (van der Vorst 1992) replacing AMGCL's BiCGSTAB
-// (src/HO_2D.hpp:53-54, src/HO_2D.cpp:1960). Preconditioner, two-level V(0,1):
-//   coarse:  e = P A1^{-1} P^T f, P = element-wise constants, A1 = P^T A P, A1^{-1}
-//            approximated by one smoothed-aggregation V-cycle (host_amg.cpp);
-//   smooth:  z = e + w D^{-1} (f - A e), D = the K^2 x K^2 diagonal blocks of A; A e is
-//            cheap because e is element-wise constant (A e = sum_s rowsum_s e_s).
-// With HO2D_PRECOND=bj the preconditioner is z = D^{-1} f (block-Jacobi).
+// (src/HO_2D.hpp:53-54, src/HO_2D.cpp:1960). Preconditioner, two-level and additive:
+//   z = P A1^{-1} R f + w D^{-1} f,
+// P = continuous bilinear interpolation from the mesh vertices, R = its transpose times the
+// quadrature weights, A1 = the bilinear finite-element Laplacian on the vertices
+// (host_amg.cpp), A1^{-1} approximated by one smoothed-aggregation V-cycle, D = the
+// K^2 x K^2 diagonal blocks of A. (Two-level methods for discontinuous schemes with this
+// coarse space: Dobrev, Lazarov, Vassilevski, Zikatanov 2006.) The vertices carry the
+// element's linear modes, which element-wise constants leave to the smoother, and because
+// P u has no jumps the sum needs no A P u: the smoothing and the coarse cycle are
+// independent, and the combination reads four values per element.
+// With HO2D_PRECOND=bj the preconditioner is z = w D^{-1} f (block-Jacobi).
 // Scalars stay on the device; every vector update fuses the dot products the next step
 // needs, reduced deterministically (per-CTA partials summed in a fixed order by the last
 // CTA to finish); a `done` flag turns the rest of an enqueued batch into no-ops, so the
@@ -162,7 +167,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_trace_in(MfOp<T> op, const
     row_emit_traces<K, T>(op.b, buf[ix.warp][ix.lw], row, dst, tv, tg, ix.t, ix.active);
 }
 
-// r = b - A x (x's traces in xtv/xtg), rhat = r; ||r||^2, ||b||^2; element sums of r. Like
+// r = b - A x (x's traces in xtv/xtg), rhat = r; ||r||^2, ||b||^2; element moments of r. Like
 // every reducing row kernel it runs as one wave of CTAs, each taking element tiles
 // blockIdx.x, blockIdx.x + gridDim.x, ... and reducing once.
 template <int K, typename T>
@@ -172,25 +177,22 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_mf_init(MfOp<T> op, BicgVe
     double part[2] = {0.0, 0.0};
     auto tile_body = [&](int tile) {
         const RowIdx<K> ix(op.g.N, tile);
-        T y[K];
+        T y[K], r[K];
         row_apply<K, T>(op, v.x, v.xtv, v.xtg, sm[ix.warp], ix, y);
-        T rsum = T(0);
         if (ix.active) {
             const size_t p = (size_t)ix.el * K * K + ix.t * K;
-            T bb[K], r[K];
+            T bb[K];
             load_row<K, T>(v.b + p, bb);
 #pragma unroll
             for (int i = 0; i < K; ++i) {
                 r[i] = bb[i] - y[i];
-                rsum += r[i];
                 part[0] += double(r[i]) * double(r[i]);
                 part[1] += double(bb[i]) * double(bb[i]);
             }
             store_row<K, T>(v.r + p, r);
             store_row<K, T>(v.rhat + p, r);
         }
-        const T tot = element_total<K, T>(rsum, ix.lw);
-        if (ix.active && ix.t == 0) v.er[ix.el] = tot;
+        element_moments<K, T>(op.h, r, sm[ix.warp].com[ix.lw], ix, v.er);
     };
     // FP32: one wave of CTAs over the tiles; FP64 keeps one tile per CTA (the loop would
     // push the operator past the register file)
@@ -441,7 +443,7 @@ struct SmootherData {
 //   mode 1:  s = r - alpha v, ||s||^2 (s_exit test),                      f = s
 // then zf = M f with the smoother's element inverse M (exact FP32/FP64 block, BF16 block or
 // Kronecker-sum factors). It needs nothing of the coarse cycle, which runs beside it on a
-// second stream; k_post_b combines the two. Mode 0 also stores the element sums of the new
+// second stream; k_post_b combines the two. Mode 0 also stores the element moments of the new
 // p for the next iteration. Row-parallel (rows.cuh): thread t of an element owns row t. The
 // warp's element data are requested first, by one bulk copy into shared memory
 // (PostRows::kStage), so the copy overlaps the vector loads.
@@ -468,9 +470,9 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_post_a(MfOp<T> op, BicgVec
         load_row<K, T>(v.v + p, vv);
         if (mode == 0) load_row<K, T>(v.p + p, pp);
     }
-    if (mode == 0 && has_coarse && act && t == 0) {
+    if (mode == 0 && has_coarse && act) {
         const F0<T> f0 = f0_of(v, sc, mode);
-        v.ep[(sc->it + 1) & 1][el] = f0[el];
+        for (int c = t; c < 4; c += K) v.ep[(sc->it + 1) & 1][el * 4 + c] = f0[el * 4 + c];
     }
     // the operand: p or s
     T f[K];
@@ -514,81 +516,51 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_post_a(MfOp<T> op, BicgVec
     }
 }
 
-// Coarse part of the preconditioner application and the result: the two-level smoothing
-// step z = e + w M (f - A e), e = P u0 element-wise constant, as
-//   z = u0_self + w (zf - sum_s W_s u0_s),   W_s = M rowsum_s  (k_make_w, at setup),
-// where A e = sum over the element's 5 block slots s (itself, its face neighbours) of the
-// block row sums times u0 of the slot's element; then z's face traces. Without a coarse
-// level (block-Jacobi) z = w zf.
+// The preconditioner application's result z = P u0 + w zf, row t of an element: the coarse
+// function is bilinear in the element, so the thread interpolates its four corner values to
+// the row's two ends and runs along the row between them. conn == nullptr: no coarse level.
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS) k_post_b(MfOp<T> op, BicgVectors<T> v, CoarseOut<T> co,
-                                                              int has_coarse, double w, const KrylovScalars* sc,
-                                                              int mode) {
+__device__ __forceinline__ void combine_row(const HatBases<T>& h, const int* __restrict__ conn,
+                                            const T* __restrict__ u0, const T* __restrict__ zf, T w, int el, int t,
+                                            T (&z)[K]) {
+    T f[K];
+    load_row<K, T>(zf, f);
+    T l = T(0), r = T(0);
+    if (conn) {
+        int c[4];
+        load4i(conn + (size_t)el * 4, c);
+        T u[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) u[q] = c[q] >= 0 ? u0[c[q]] : T(0);
+        const T y0 = h.hp[t * 2 + 0], y1 = h.hp[t * 2 + 1];
+        l = u[0] * y0 + u[3] * y1;
+        r = u[1] * y0 + u[2] * y1;
+    }
+#pragma unroll
+    for (int i = 0; i < K; ++i) z[i] = (l * h.hp[i * 2 + 0] + r * h.hp[i * 2 + 1]) + w * f[i];
+}
+
+// z of the preconditioner application and its face traces. Bound by HBM: zf read, z and the
+// two trace buffers written; the four corner values are L2 reads shared by an element's
+// threads.
+template <int K, typename T>
+__global__ void __launch_bounds__(Rows<K>::THREADS) k_post_b(MfOp<T> op, BicgVectors<T> v,
+                                                              const int* __restrict__ conn,
+                                                              const T* __restrict__ u0, double w,
+                                                              const KrylovScalars* sc, int mode) {
     using R = Rows<K>;
-    constexpr int K2 = R::K2;
     if (sc->done) return;  // uniform
     __shared__ T zb[R::WARPS][R::EPW][K][K];
     const RowIdx<K> ix(op.g.N, blockIdx.x);
-    const int t = ix.t, el = ix.el;
-    const bool act = ix.active;
-    const size_t p = (size_t)el * K2 + t * K;
+    const size_t p = (size_t)ix.el * R::K2 + ix.t * K;
     T zz[K];
     int dst[4];
-    if (act) {
-        T zf[K];
-        load_row<K, T>(v.zf + p, zf);
-        load4i(op.g.scat + ((size_t)el * K + t) * 4, dst);
-        T ue[5], ws[5][K];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            ue[q] = has_coarse ? co.ue5[(size_t)el * 5 + q] : T(0);
-            if (has_coarse) load_row<K, T>(op.W + ((size_t)el * 5 + q) * K2 + t * K, ws[q]);
-        }
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-            T ae = T(0);
-            if (has_coarse) {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) ae += ws[q][i] * ue[q];
-            }
-            zz[i] = ue[0] + T(w) * (zf[i] - ae);
-        }
+    if (ix.active) {
+        load4i(op.g.scat + ((size_t)ix.el * K + ix.t) * 4, dst);
+        combine_row<K, T>(op.h, conn, u0, v.zf + p, T(w), ix.el, ix.t, zz);
         store_row<K, T>((mode == 0 ? v.ph : v.sh) + p, zz);
     }
-    row_emit_traces<K, T>(op.b, zb[ix.warp][ix.lw], zz, dst, v.tv, v.tg, t, act);
-}
-
-// Setup: W_s = M rowsum_s for the 5 block slots of every element, with the smoother's own
-// element inverse M (so the split application k_post_a + k_post_b is exactly the smoothing
-// step of the stored smoother).
-template <int K, typename T, int BS>
-__global__ void __launch_bounds__(Rows<K>::THREADS) k_make_w(MfOp<T> op, T* __restrict__ W, KrylovScalars* sc) {
-    using R = Rows<K>;
-    constexpr int K2 = R::K2, EPW = R::EPW;
-    extern __shared__ __align__(128) unsigned char post_dyn[];
-    __shared__ __align__(8) uint64_t bar[R::WARPS];
-    __shared__ __align__(16) T sr[R::WARPS][EPW][K2];
-    __shared__ T zb[R::WARPS][EPW][K][K];
-    const RowIdx<K> ix(op.g.N, blockIdx.x);
-    const int t = ix.t, lw = ix.lw, el = ix.el;
-    const bool act = ix.active;
-    SmootherData<K, T, BS> sd;
-    sd.start(op, ix, post_dyn, &bar[ix.warp], true);
-    sd.wait(&bar[ix.warp], sc, ix.lane);
-    for (int q = 0; q < 5; ++q) {
-        const size_t rq = ((size_t)el * 5 + q) * K2 + t * K;
-        if (act) {
-            T r[K];
-            load_row<K, T>(op.rowsum + rq, r);
-#pragma unroll
-            for (int i = 0; i < K; ++i) sr[ix.warp][lw][t * K + i] = r[i];
-        }
-        __syncwarp();
-        T acc[K];
-        smoother_rows<K, T, BS>(op, sd.blk, sd.fk, sd.kx, sr[ix.warp][lw], zb[ix.warp][lw], t, act, acc);
-        if (act) store_row<K, T>(W + rq, acc);
-        __syncwarp();  // sr is rewritten for the next slot
-    }
+    row_emit_traces<K, T>(op.b, zb[ix.warp][ix.lw], zz, dst, v.tv, v.tg, ix.t, ix.active);
 }
 
 // The FP32 operator's tile loop with its inputs staged in shared memory (apply_stage.cuh):
@@ -642,7 +614,7 @@ __device__ __forceinline__ void staged_apply_loop(const MfOp<float>& op, const f
     }
 }
 
-// v = A ph; alpha = rho / (rhat, v); element sums of v. ST: the FP32 loop with staged
+// v = A ph; alpha = rho / (rhat, v); element moments of v. ST: the FP32 loop with staged
 // inputs (dynamic shared memory ApplyStage<K>::CTA_BYTES).
 // (FP32: at most 128 registers, four CTAs per SM)
 template <int K, typename T, bool ST = false>
@@ -656,18 +628,13 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 1)
     const int ntiles = (int)rgrid_of<K>(op.g.N);
     double part[1] = {0.0};
     auto finish = [&](const RowIdx<K>& ix, const T (&y)[K], const T (&rh)[K]) {
-        T ysum = T(0);
         if (ix.active) {
             const size_t p = (size_t)ix.el * K * K + ix.t * K;
             store_row<K, T>(v.v + p, y);
 #pragma unroll
-            for (int i = 0; i < K; ++i) {
-                ysum += y[i];
-                part[0] += double(rh[i]) * double(y[i]);
-            }
+            for (int i = 0; i < K; ++i) part[0] += double(rh[i]) * double(y[i]);
         }
-        const T tot = element_total<K, T>(ysum, ix.lw);
-        if (ix.active && ix.t == 0) v.ev[ix.el] = tot;
+        element_moments<K, T>(op.h, y, sm[ix.warp].com[ix.lw], ix, v.ev);
     };
     auto tile_body = [&](int tile) {
         const RowIdx<K> ix(op.g.N, tile);
@@ -750,7 +717,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 1)
         sc->omega = out[1] > 0.0 ? out[0] / out[1] : 0.0;
 }
 
-// x += alpha ph + omega sh; r = s - omega t; ||r||^2, (rhat, r); element sums of r;
+// x += alpha ph + omega sh; r = s - omega t; ||r||^2, (rhat, r); element moments of r;
 // convergence test. After an s-exit (||s|| already below tolerance) only x += alpha ph.
 // The last CTA to finish ends the iteration: it updates the scalars, sets `done`, and
 // inside a captured solve sets the condition of the graph's while node (iterate while
@@ -759,9 +726,10 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 1)
 // max_iter) or finds `done` set and clears the condition, so the device loop always ends.
 // Each thread updates element rows.
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, BicgVectors<T> v, ReduceScratch rs,
-                                                                 int max_iter, cudaGraphConditionalHandle h,
-                                                                 int has_handle) {
+__global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, HatBases<T> hats, BicgVectors<T> v,
+                                                                 ReduceScratch rs, int max_iter,
+                                                                 cudaGraphConditionalHandle h, int has_handle) {
+    __shared__ T mom[Rows<K>::WARPS][Rows<K>::EPW][4][K];
     KrylovScalars* sc = rs.sc;
     if (sc->done) {  // the solve ended earlier in this body (breakdown)
         if (has_handle && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
@@ -776,7 +744,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, BicgVecto
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const RowIdx<K> ix(N, tile);
         const size_t p = (size_t)ix.el * K * K + ix.t * K;
-        T rsum = T(0);
+        T r[K];
         if (ix.active) {
             T x[K], ph[K];
             load_row<K, T>(v.x + p, x);
@@ -786,7 +754,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, BicgVecto
                 for (int i = 0; i < K; ++i) x[i] = x[i] + alpha * ph[i];
                 store_row<K, T>(v.x + p, x);
             } else {
-                T sh[K], sv[K], tv[K], rh[K], r[K];
+                T sh[K], sv[K], tv[K], rh[K];
                 load_row<K, T>(v.sh + p, sh);
                 load_row<K, T>(v.s + p, sv);
                 load_row<K, T>(v.t + p, tv);
@@ -795,7 +763,6 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, BicgVecto
                 for (int i = 0; i < K; ++i) {
                     x[i] = x[i] + (alpha * ph[i] + T(omega) * sh[i]);
                     r[i] = sv[i] - T(omega) * tv[i];
-                    rsum += r[i];
                     part[0] += double(r[i]) * double(r[i]);
                     part[1] += double(rh[i]) * double(r[i]);
                 }
@@ -803,10 +770,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, BicgVecto
                 store_row<K, T>(v.r + p, r);
             }
         }
-        if (!s_exit) {
-            const T tot = element_total<K, T>(rsum, ix.lw);
-            if (ix.active && ix.t == 0) v.er[ix.el] = tot;
-        }
+        if (!s_exit) element_moments<K, T>(hats, r, mom[ix.warp][ix.lw], ix, v.er);
     }
     double out[2];
     if (grid_reduce<2>(part, rs.partials, rs.counter, out) && threadIdx.x == 0) {
@@ -819,6 +783,9 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, BicgVecto
             sc->rho_old = sc->rho;
             sc->rho = out[1];
             if (out[0] <= sc->eps2 || sc->it >= max_iter || omega == 0.0) sc->done = 1;
+            // an FP32 solve whose residual has grown a millionfold is lost (krylov_usable
+            // then drops its result)
+            if (sizeof(T) == 4 && !(out[0] <= 1e12 * sc->bnorm2)) sc->done = 1;
         }
         if (has_handle) cudaGraphSetConditional(h, sc->done ? 0u : 1u);
     }
@@ -934,10 +901,12 @@ __global__ void k_refine_prep(const double* __restrict__ r, float* __restrict__ 
     }
 }
 
-// psi += x; the inner iterations are added to the solve's total
+// psi += x; the inner iterations are added to the solve's total. An inner solve that broke
+// down adds nothing: the residual stays, which the decision after it takes for a stall, and
+// the FP64 solve goes on from psi.
 __global__ void k_refine_axpy(const float* __restrict__ e, double* __restrict__ x, size_t n, KrylovScalars* sc) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) x[i] += (double)e[i];
+    if (i < n && krylov_usable(*sc)) x[i] += (double)e[i];
     if (i == 0) sc->iters_total += sc->it;
 }
 
@@ -1006,7 +975,6 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
     };
     const int N = op.g.N;
     const int mg = pc.nlev > 0;
-    const CoarseOut<T> co = mg ? coarse_out(pc) : CoarseOut<T>();
     const unsigned gp = rgrid_of<K>(N);
     constexpr int tp = Rows<K>::THREADS;
     auto post_a = [&](int mode) {
@@ -1039,7 +1007,7 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
         post_a(mode);
         if (fork) cudaStreamWaitEvent(s, op.ev_join, 0);
         mark(m0 + 2);
-        k_post_b<K, T><<<gp, tp, 0, s>>>(op, v, co, mg, pc.omega, rs.sc, mode);
+        k_post_b<K, T><<<gp, tp, 0, s>>>(op, v, mg ? pc.conn : nullptr, pc.lev[0].u, pc.omega, rs.sc, mode);
     };
     const unsigned gwv = wave_of<K, T>(&WaveSizes::v, N), gwt = wave_of<K, T>(&WaveSizes::t, N),
                    gwx = wave_of<K, T>(&WaveSizes::xr, N);
@@ -1071,7 +1039,7 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
     mark(7);
     apply_t();
     mark(8);
-    k_xr_update<K, T><<<gwx, Rows<K>::THREADS, 0, s>>>(N, v, rs, max_iter, h, has_handle);
+    k_xr_update<K, T><<<gwx, Rows<K>::THREADS, 0, s>>>(N, op.h, v, rs, max_iter, h, has_handle);
     mark(9);
 }
 
@@ -1111,10 +1079,6 @@ static cudaError_t configure_post() {
     one(k_post_a<K, float, 0>, PostRows<K, float, 0>::SMEM);
     one(k_post_a<K, float, 1>, PostRows<K, float, 1>::SMEM);
     one(k_post_a<K, float, 2>, PostRows<K, float, 2>::SMEM);
-    one(k_make_w<K, double, 0>, PostRows<K, double, 0>::SMEM);
-    one(k_make_w<K, float, 0>, PostRows<K, float, 0>::SMEM);
-    one(k_make_w<K, float, 1>, PostRows<K, float, 1>::SMEM);
-    one(k_make_w<K, float, 2>, PostRows<K, float, 2>::SMEM);
     return e;
 }
 
@@ -1129,31 +1093,6 @@ cudaError_t krylov_configure(int K) {
 template <typename T>
 int krylov_launches_per_iteration(const Precond<T>& pc) {
     return 7 + 2 * coarse_launches(pc);
-}
-
-template <int K, typename T>
-static cudaError_t make_w_impl(const MfOp<T>& op, T* W, KrylovScalars* sc, cudaStream_t s) {
-    const unsigned g = rgrid_of<K>(op.g.N);
-    constexpr int tp = Rows<K>::THREADS;
-    if constexpr (std::is_same<T, float>::value) {
-        if (op.kron_f) {
-            k_make_w<K, T, 2><<<g, tp, PostRows<K, T, 2>::SMEM, s>>>(op, W, sc);
-            return cudaGetLastError();
-        }
-        if (op.dinv_bf16) {
-            k_make_w<K, T, 1><<<g, tp, PostRows<K, T, 1>::SMEM, s>>>(op, W, sc);
-            return cudaGetLastError();
-        }
-    }
-    k_make_w<K, T, 0><<<g, tp, PostRows<K, T, 0>::SMEM, s>>>(op, W, sc);
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t krylov_make_w(const MfOp<T>& op, T* W, KrylovScalars* sc, cudaStream_t s) {
-    cudaError_t e = cudaSuccess;
-    HO2D_KSWITCH(op.K, (e = make_w_impl<KK, T>(op, W, sc, s)));
-    return e;
 }
 
 template <typename T>
@@ -1329,7 +1268,6 @@ cudaError_t launch_axpy_f2d(const float* e, double* x, size_t n, cudaStream_t s)
     template cudaError_t krylov_iteration<T>(const MfOp<T>&, const BicgVectors<T>&, const ReduceScratch&, int,    \
                                              const Precond<T>&, cudaStream_t);                                    \
     template int krylov_launches_per_iteration<T>(const Precond<T>&);                                             \
-    template cudaError_t krylov_make_w<T>(const MfOp<T>&, T*, KrylovScalars*, cudaStream_t);                      \
     template cudaError_t krylov_iteration_timed<T>(const MfOp<T>&, const BicgVectors<T>&, const ReduceScratch&,   \
                                                    int, const Precond<T>&, cudaEvent_t*, cudaStream_t);           \
     template cudaError_t krylov_capture_solve<T>(const MfOp<T>&, const BicgVectors<T>&, const ReduceScratch&,     \

@@ -215,14 +215,37 @@ __device__ __forceinline__ void col_to_row(T (&buf)[K][K], const T (&col)[K], T 
     }
 }
 
-// Sum of one value over the K threads of each element, in the fixed order t = 0..K-1,
-// returned to every thread of the element. Warp-collective.
+// The element's values tested with its four hats (HatBases::hr), corners in the order
+// (-,-), (+,-), (+,+), (-,+): thread t puts its row's share of each into buf, then thread
+// c < 4 adds the K shares of corner c in the order t = 0..K-1 and stores out[4 el + c].
+// Warp-collective; a barrier separates the reads from the caller's next use of buf.
 template <int K, typename T>
-__device__ __forceinline__ T element_total(T v, int lw) {
-    T s = T(0);
+__device__ __forceinline__ void element_moments(const HatBases<T>& h, const T (&row)[K], T (&buf)[4][K],
+                                                const RowIdx<K>& ix, T* __restrict__ out) {
+    const int t = ix.t;
+    if (ix.active) {
+        T m0 = T(0), m1 = T(0);
 #pragma unroll
-    for (int m = 0; m < K; ++m) s += __shfl_sync(0xffffffffu, v, lw * K + m);
-    return s;
+        for (int i = 0; i < K; ++i) {
+            m0 += row[i] * h.hr[i * 2 + 0];
+            m1 += row[i] * h.hr[i * 2 + 1];
+        }
+        const T y0 = h.hr[t * 2 + 0], y1 = h.hr[t * 2 + 1];
+        buf[0][t] = m0 * y0;
+        buf[1][t] = m1 * y0;
+        buf[2][t] = m1 * y1;
+        buf[3][t] = m0 * y1;
+    }
+    __syncwarp();
+    if (ix.active) {
+        for (int c = t; c < 4; c += K) {
+            T s = T(0);
+#pragma unroll
+            for (int m = 0; m < K; ++m) s += buf[c][m];
+            out[(size_t)ix.el * 4 + c] = s;
+        }
+    }
+    __syncwarp();
 }
 
 // What one thread of the operator reads for its row t of element `el`: rows and columns

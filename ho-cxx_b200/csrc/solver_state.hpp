@@ -87,14 +87,13 @@ struct DeviceState {
     DeviceBuffer w_stage64;
     // Poisson operator and Krylov workspace
     // Poisson operator: matrix-free; block-Jacobi inverses and block row sums from setup
-    DeviceBuffer dinv64, dinv32, rowsum64, rowsum32, bcol;
+    DeviceBuffer dinv64, dinv32, rowsum64, bcol;
     DeviceBuffer colsum64;  // block column sums (device assembly only)
     VtkDevice vtk;
-    DeviceBuffer W64, W32, zf;  // smoother applied to the block row sums; fine part of z
-    // level-0 coarse values per element slot (one buffer per precision: the cycle writes only
-    // the slots that have a block neighbour, so a shared buffer would leave the other
-    // precision's bytes in the rest), and where each value goes
-    DeviceBuffer ue5, ue5_32, u0dst;
+    DeviceBuffer zf;         // fine part of z
+    DeviceBuffer conn, v2e;  // the coarse space's tables (Precond)
+    HatBases<double> hat64;
+    HatBases<float> hat32;
     DeviceBuffer dinv_bf16;  // BF16 copy of dinv for the FP32 smoother (HO2D_SMOOTHER_BF16=1)
     // Kronecker-sum smoother for the FP32 solve (HO2D_SMOOTHER_KRON=1): factors, exact-block
     // index per element, compact exact blocks
@@ -106,7 +105,7 @@ struct DeviceState {
     // FP32 operator inputs staged by bulk copies (HO2D_OP_STAGE=1) instead of read through
     // L2 prefetches (the default: 51 against 60 us per launch on the 256 x 512 O-grid, K = 6)
     bool op_staged = false;
-    DeviceBuffer esum[4];  // element sums of r, v, p (two alternating buffers), N + 4 entries
+    DeviceBuffer esum[4];  // element moments [N][4] of r, v, p (two alternating buffers)
     DeviceBuffer ktv, ktg, kxtv, kxtg;  // face traces of the Krylov operand and of x
     DeviceBuffer partials, counter, scalars;
     KrylovScalars* h_sc = nullptr;
@@ -295,9 +294,7 @@ MfOp<T> make_op(DeviceState& d, const Mesh& m, int K, bool f32) {
     op.kron_f = kron ? (const T*)d.kron_f.get() : nullptr;
     op.kron_x = kron ? d.kron_x.as<int>() : nullptr;
     op.kron_exact = kron ? (const T*)d.kron_exact.get() : nullptr;
-    op.rowsum = f32 ? (const T*)d.rowsum32.get() : (const T*)d.rowsum64.get();
-    op.bcol = d.bcol.as<int>();
-    op.W = f32 ? (const T*)d.W32.get() : (const T*)d.W64.get();
+    op.h = *reinterpret_cast<const HatBases<T>*>(f32 ? (const void*)&d.hat32 : (const void*)&d.hat64);
     op.staged = f32 && d.op_staged ? 1 : 0;
     op.side = d.side;
     op.ev_fork = d.ev_fork;
