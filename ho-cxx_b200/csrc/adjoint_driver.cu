@@ -53,35 +53,11 @@ Tableau tableau(int ti_type) {
     return t;
 }
 
-Csr transpose_csr(const Csr& A) {
-    Csr T;
-    T.n = A.m;
-    T.m = A.n;
-    T.ptr.assign((size_t)T.n + 1, 0);
-    for (int c : A.col) ++T.ptr[(size_t)c + 1];
-    for (int i = 0; i < T.n; ++i) T.ptr[(size_t)i + 1] += T.ptr[i];
-    T.col.resize(A.col.size());
-    T.val.resize(A.val.size());
-    std::vector<int> pos(T.ptr.begin(), T.ptr.end() - 1);
-    for (int r = 0; r < A.n; ++r)
-        for (int q = A.ptr[r]; q < A.ptr[(size_t)r + 1]; ++q) {
-            const int dst = pos[A.col[q]]++;
-            T.col[dst] = r;
-            T.val[dst] = A.val[q];
-        }
-    return T;
-}
-
-template <typename T>
-const DevBases<T>& bases_of(const DeviceState& d, bool f32) {
-    return *reinterpret_cast<const DevBases<T>*>(f32 ? (const void*)&d.b32 : (const void*)&d.b64);
-}
-
 }  // namespace
 
 int Solver::adjoint_steps() const { return adj_ ? adj_->nsteps : -1; }
 
-// Buffers and the preconditioner of the transposed Poisson problem, built once per setup.
+// Buffers of the adjoint, allocated once per setup.
 Error Solver::adjoint_prepare() {
     if (!setup_done_) return {1, "call ho2d_setup first"};
     if (!adj_) adj_.reset(new AdjointState);
@@ -101,87 +77,54 @@ Error Solver::adjoint_prepare() {
     for (DeviceBuffer* b : {&a.sv, &a.sg, &a.swv, &a.swg, &a.sU, &a.spv, &a.spg})
         HO2D_CUDA(upload(*b, zf), "alloc adjoint slots");
     for (DeviceBuffer* b : {&a.lbc_d, &a.lbc_nv, &a.lpv}) HO2D_CUDA(upload(*b, zb), "alloc adjoint boundary");
-    HO2D_CUDA(upload(a.f0, std::vector<double>((size_t)N + 4, 0.0)), "alloc element sums");
-    HO2D_CUDA(upload(a.partials, std::vector<double>((size_t)2 * kt_grid(), 0.0)), "alloc partials");
-    HO2D_CUDA(upload(a.counter, std::vector<unsigned>(1, 0u)), "alloc counter");
-    HO2D_CUDA(a.scalars.alloc(sizeof(KrylovScalars)), "alloc scalars");
-    HO2D_CUDA(cudaMemset(a.scalars.get(), 0, sizeof(KrylovScalars)), "memset");
-    // column sums of A's blocks: (A^T P u)(el, ij) = sum over the 5 block slots of el of
-    // u[c] * sum_r A[(c, r), (el, ij)], c = the slot's element: the column sums (over rows
-    // r, ascending) of block (c, s2), the slot of c whose column element is el
-    HO2D_TRY(ensure_host_colsum());
-    std::vector<double> rsT((size_t)N * 5 * K2, 0.0);
-    for (int el = 0; el < N; ++el)
-        for (int s = 0; s < 5; ++s) {
-            const int c = op_.block_col[(size_t)el * 5 + s];
-            if (c < 0) continue;
-            int s2 = -1;
-            for (int q = 0; q < 5; ++q)
-                if (op_.block_col[(size_t)c * 5 + q] == el) s2 = q;
-            if (s2 < 0) return {3, "Poisson block structure is not symmetric"};
-            const double* cs = &op_.colsum[((size_t)c * 5 + s2) * K2];
-            std::copy(cs, cs + K2, rsT.begin() + ((size_t)el * 5 + s) * K2);
-        }
-    HO2D_CUDA(upload(a.rowsumT64, rsT), "upload transposed row sums");
-    HO2D_CUDA(upload_as<float>(a.rowsumT32, rsT), "upload transposed row sums");
-    // coarse hierarchy of the transposed P0 problem (same settings as the forward one)
-    a.pc64 = Precond<double>();
-    a.pc32 = Precond<float>();
-    a.lev.clear();
-    const char* mode = std::getenv("HO2D_PRECOND");
-    const char* om = std::getenv("HO2D_MG_OMEGA");
-    const double omega = om ? std::atof(om) : 0.7;
-    a.pc64.omega = a.pc32.omega = omega;
-    if (!(mode && std::string(mode) == "bj")) {
-        const char* dm = std::getenv("HO2D_DENSE_MAX");
-        const int dmax = dm ? std::max(1, std::atoi(dm)) : kDenseMax;
-        CoarseHierarchy H;
-        HO2D_TRY(build_coarse_hierarchy(transpose_csr(p0_coarse_operator(op_, N)), H, dmax, dm ? dmax : kDenseMaxFirst,
-                                        !device_setup_));
-        HO2D_TRY(upload_hierarchy(H, omega, a.lev, a.dense64, a.dense32, a.pc64, a.pc32, nullptr));
-    }
     HO2D_CUDA(cudaDeviceSynchronize(), "adjoint setup");
     a.ready = true;
     return {0, ""};
 }
 
-// BiCGSTAB on A^T x = b in precision T to relative tolerance tol; x starts at zero.
+// BiCGSTAB on A^T x = b in precision T to relative tolerance tol; x starts at zero. The
+// forward solver's iteration (krylov.cu) on the transposed operator: D^-T for D^-1, and the
+// coarse space's interpolation and restriction exchanged.
 template <typename T>
 Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
     DeviceState& d = *d_;
     AdjointState& a = *adj_;
-    const int K = in_.knod;
-    const size_t n = (size_t)mesh_.n_el * K * K;
-    TVectors<T> v;
-    v.x = x;
-    v.r = a.kv[0].as<T>();
-    v.rhat = a.kv[1].as<T>();
-    v.p = a.kv[2].as<T>();
-    v.v = a.kv[3].as<T>();
-    v.s = a.kv[4].as<T>();
-    v.t = a.kv[5].as<T>();
-    v.ph = a.kv[6].as<T>();
-    v.sh = a.kv[7].as<T>();
-    v.dir = a.kv[8].as<T>();
-    v.b = b;
-    v.sv = a.sv.as<T>();
-    v.sg = a.sg.as<T>();
-    v.f0 = a.f0.as<T>();
-    TPrecond<T> pc;
-    pc.pc = *reinterpret_cast<const Precond<T>*>(f32 ? (const void*)&a.pc32 : (const void*)&a.pc64);
-    pc.dinv = f32 ? (const T*)d.dinv32.get() : (const T*)d.dinv64.get();
-    pc.rowsumT = f32 ? (const T*)a.rowsumT32.get() : (const T*)a.rowsumT64.get();
-    pc.bcol = d.bcol.as<int>();
-    const TReduce red{a.partials.as<double>(), a.counter.as<unsigned>(), a.scalars.as<KrylovScalars>()};
-    const FrGeom<T> g = geom_of<T>(d, mesh_, f32);
-    const DevBases<T>& bb = bases_of<T>(d, f32);
-    // the element sums' padding and the boundary entries of the slots must read as zero in
-    // precision T; these buffers are shared by the FP64 and FP32 solves
-    HO2D_CUDA(cudaMemsetAsync(a.f0.get(), 0, a.f0.bytes(), d.stream), "memset");
+    const int N = mesh_.n_el, K = in_.knod;
+    DeviceBuffer& dinvT = f32 ? a.dinvT32 : a.dinvT64;
+    MfOp<T> op = make_op<T>(d, mesh_, K, f32);
+    if (!dinvT.get()) {
+        HO2D_CUDA(dinvT.alloc(((size_t)N * padded_count(K * K * K * K, (int)sizeof(T)) + 1) * sizeof(T)),
+                  "alloc transposed blocks");
+        HO2D_CUDA(cudaMemsetAsync(dinvT.get(), 0, dinvT.bytes(), d.stream), "memset");
+        HO2D_CUDA(transpose_blocks<T>(N, K, op.dinv, dinvT.as<T>(), d.stream), "transposed blocks");
+        launches_ += 1;
+    }
+    op.transposed = 1;
+    op.dinv = dinvT.as<T>();
+    op.dinv_bf16 = nullptr;
+    op.kron_f = op.kron_exact = nullptr;
+    op.kron_x = nullptr;
+    op.staged = 0;
+    std::swap(op.h.hp, op.h.hr);
+    BicgVectors<T> v = krylov_vectors<T>(d, x, b);
+    T** kv[8] = {&v.r, &v.rhat, &v.p, &v.v, &v.s, &v.t, &v.ph, &v.sh};
+    for (int i = 0; i < 8; ++i) *kv[i] = a.kv[i].as<T>();
+    v.tv = a.sv.as<T>();
+    v.tg = a.sg.as<T>();
+    const Precond<T>& pc = *reinterpret_cast<const Precond<T>*>(f32 ? (const void*)&d.pc32 : (const void*)&d.pc64);
+    const ReduceScratch rs{d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>()};
+    // the boundary entries of the slots must read as zero in precision T; the FP64 and FP32
+    // solves share these buffers
     HO2D_CUDA(cudaMemsetAsync(a.sv.get(), 0, a.sv.bytes(), d.stream), "memset");
     HO2D_CUDA(cudaMemsetAsync(a.sg.get(), 0, a.sg.bytes(), d.stream), "memset");
     d.h_sc->tol = tol;  // the stream is idle: the last read of h_sc was synchronised
-    HO2D_CUDA(cudaMemcpyAsync(&red.sc->tol, &d.h_sc->tol, sizeof(double), cudaMemcpyHostToDevice, d.stream), "tol");
+    HO2D_CUDA(cudaMemcpyAsync(&rs.sc->tol, &d.h_sc->tol, sizeof(double), cudaMemcpyHostToDevice, d.stream), "tol");
+    auto poll = [&]() -> Error {
+        HO2D_CUDA(cudaMemcpyAsync(d.h_sc, rs.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, d.stream), "poll");
+        HO2D_CUDA(cudaStreamSynchronize(d.stream), "poll");
+        if (d.h_sc->dev_error) return {5, "a device-side wait for a bulk copy ran out (the GPU did not complete it)"};
+        return {0, ""};
+    };
     if (use_graphs_) {
         // one launch of the captured solve (init and a device-side while loop); the graph
         // bakes in the operands, so it is recaptured when they change
@@ -189,31 +132,30 @@ Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
         SolveGraph& sg = a.graph[gi];
         if (!sg.exec || sg.max_iter != max_iter_ || a.graph_x[gi] != (const void*)x || a.graph_b[gi] != (const void*)b) {
             sg.reset();
-            HO2D_CUDA(kt_capture_solve<T>(K, g, bb, v, pc, red, max_iter_, d.stream, &sg.graph), "graph capture");
-            HO2D_CUDA(cudaGraphInstantiate(&sg.exec, sg.graph, 0), "graph instantiate");
+            HO2D_CUDA(krylov_capture_solve<T>(op, v, rs, max_iter_, pc, d.stream, &sg.graph), "graph capture");
+            HO2D_CUDA(cudaGraphInstantiate(&sg.exec, sg.graph, cudaGraphInstantiateFlagUseNodePriority),
+                      "graph instantiate");
             sg.max_iter = max_iter_;
             a.graph_x[gi] = x;
             a.graph_b[gi] = b;
         }
         HO2D_CUDA(cudaGraphLaunch(sg.exec, d.stream), "graph launch");
-        HO2D_CUDA(cudaMemcpyAsync(d.h_sc, red.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, d.stream), "poll");
-        HO2D_CUDA(cudaStreamSynchronize(d.stream), "poll");
+        HO2D_TRY(poll());
         iters = d.h_sc->it;
-        launches_ += 2 + (int64_t)iters * kt_launches_per_iteration<T>(pc);
+        launches_ += 2 + (int64_t)iters * krylov_launches_per_iteration(pc);
         return {0, ""};
     }
-    HO2D_CUDA(kt_init<T>(n, v, red, d.stream), "transposed init");
+    HO2D_CUDA(krylov_init<T>(op, v, rs, d.stream), "transposed init");
     launches_ += 1;
     // batches of iterations between polls of the done flag; an iteration enqueued after
     // the solve finished returns at once in every kernel
     int chunk = std::max(1, adj_prev_iters_ - 1);
     for (;;) {
         for (int c = 0; c < chunk; ++c) {
-            HO2D_CUDA(kt_iteration<T>(K, g, bb, v, pc, red, max_iter_, d.stream), "transposed iteration");
-            launches_ += kt_launches_per_iteration<T>(pc);
+            HO2D_CUDA(krylov_iteration<T>(op, v, rs, max_iter_, pc, d.stream), "transposed iteration");
+            launches_ += krylov_launches_per_iteration(pc);
         }
-        HO2D_CUDA(cudaMemcpyAsync(d.h_sc, red.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, d.stream), "poll");
-        HO2D_CUDA(cudaStreamSynchronize(d.stream), "poll");
+        HO2D_TRY(poll());
         if (d.h_sc->done) break;
         chunk = 2;
     }
@@ -229,7 +171,7 @@ Error Solver::transposed_solve(const double* rhs, double* mu) {
     AdjointState& a = *adj_;
     const int N = mesh_.n_el, K = in_.knod;
     const size_t nv = (size_t)N * K * K;
-    const TReduce red{a.partials.as<double>(), a.counter.as<unsigned>(), a.scalars.as<KrylovScalars>()};
+    const ReduceScratch rs{d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>()};
     bool finite = true;
     last_adj_iters_ = 0;
     int sweeps = 0;
@@ -241,30 +183,46 @@ Error Solver::transposed_solve(const double* rhs, double* mu) {
         finite = std::isfinite(bn) && std::isfinite(rn);
         last_adj_res_ = bn > 0 ? std::sqrt(rn / bn) : 0.0;
     } else {
-        const FrGeom<double> g = geom_of<double>(d, mesh_, false);
+        const MfOp<double> op = make_op<double>(d, mesh_, K, false);
         HO2D_CUDA(cudaMemsetAsync(mu, 0, nv * 8, d.stream), "memset");
+        double prev = 0.0;
+        bool lost = false;
         for (;; ++sweeps) {
             HO2D_CUDA(cudaMemsetAsync(a.sv.get(), 0, a.sv.bytes(), d.stream), "memset");  // shared with FP32
             HO2D_CUDA(cudaMemsetAsync(a.sg.get(), 0, a.sg.bytes(), d.stream), "memset");
-            HO2D_CUDA(poisson_transpose<double>(K, g, d.b64, mu, a.kv[9].as<double>(), a.kv[8].as<double>(),
-                                                a.sv.as<double>(), a.sg.as<double>(), nullptr, 0, d.stream),
-                      "transposed operator");
-            HO2D_CUDA(kt_residual<double>(nv, rhs, a.kv[9].as<double>(), a.res64.as<double>(), red, d.stream),
+            HO2D_CUDA(mf_apply_transpose<double>(op, mu, a.kv[0].as<double>(), a.sv.as<double>(), a.sg.as<double>(), nullptr,
+                                                 rhs, a.res64.as<double>(), rs, d.stream),
                       "transposed residual");
-            launches_ += 3;
-            HO2D_CUDA(cudaMemcpyAsync(d.h_sc, red.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, d.stream), "poll");
+            launches_ += 2;
+            HO2D_CUDA(cudaMemcpyAsync(d.h_sc, rs.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, d.stream), "poll");
             HO2D_CUDA(cudaStreamSynchronize(d.stream), "poll");
             const double bn = d.h_sc->bnorm2, rn = d.h_sc->rnorm2;
             finite = std::isfinite(bn) && std::isfinite(rn);
             last_adj_res_ = bn > 0 ? std::sqrt(rn / bn) : 0.0;
             if (!finite || bn == 0.0) break;
             if (rn <= tol_ * tol_ * bn || sweeps >= 30) break;
+            // a sweep that did not halve the residual (the forward refinement's rule) or an FP32
+            // solve that broke down: the FP64 solve of the remaining residual finishes
+            if (lost || (sweeps > 0 && !(last_adj_res_ <= 0.5 * prev))) {
+                int it = 0;
+                HO2D_TRY(kt_run<double>(a.x32.as<double>(), a.res64.as<double>(), false,
+                                        std::min(0.5, tol_ / last_adj_res_), it));
+                last_adj_iters_ += it;
+                last_adj_res_ *= std::sqrt(d.h_sc->rnorm2 / d.h_sc->bnorm2);
+                finite = std::isfinite(last_adj_res_);
+                HO2D_CUDA(launch_axpby(nv, mu, 1.0, mu, 1.0, a.x32.as<double>(), d.stream), "axpy");
+                launches_ += 1;
+                break;
+            }
+            prev = last_adj_res_;
             HO2D_CUDA(launch_copy_d2f(a.res64.as<double>(), a.b32.as<float>(), nv, d.stream), "d2f");
             const double need = 0.3 * tol_ / last_adj_res_;
             const double itol = std::min(0.5, std::max(inner_tol_, need));
             int it = 0;
             HO2D_TRY(kt_run<float>(a.x32.as<float>(), a.b32.as<float>(), true, itol, it));
             last_adj_iters_ += it;
+            lost = !krylov_usable(*d.h_sc);
+            if (lost) continue;
             HO2D_CUDA(launch_axpy_f2d(a.x32.as<float>(), mu, nv, d.stream), "axpy");
             launches_ += 2;
         }
@@ -312,7 +270,7 @@ Error Solver::stage_adjoint_dev(double coeff, double* out) {
     HO2D_CUDA(launch_residual_adjoint<double>(K, g, d.b64, sa, d.stream), "residual adjoint");
     HO2D_CUDA(launch_velocity_adjoint<double>(K, g, d.b64, sa, d.stream), "velocity adjoint");
     HO2D_CUDA(launch_gather<double>(K, N, d.b64, a.lpsi_dir.as<double>(), a.spv.as<double>(), a.spg.as<double>(),
-                                    a.lpsi.as<double>(), nullptr, 0, d.stream),
+                                    a.lpsi.as<double>(), d.stream),
               "psi gather");
     launches_ += 3;
     // psi = A^-1 (-J omega - boundary terms): lam of omega -= J A^-T lam of psi
@@ -366,10 +324,10 @@ Error Solver::apply_poisson_transpose(const double* x, double* y) {
     HO2D_CUDA(cudaMemcpyAsync(a.lpsi.get(), x, nv * 8, cudaMemcpyHostToDevice, d.stream), "copy");
     HO2D_CUDA(cudaMemsetAsync(a.sv.get(), 0, a.sv.bytes(), d.stream), "memset");  // shared with FP32
     HO2D_CUDA(cudaMemsetAsync(a.sg.get(), 0, a.sg.bytes(), d.stream), "memset");
-    const FrGeom<double> g = geom_of<double>(d, mesh_, false);
-    HO2D_CUDA(poisson_transpose<double>(in_.knod, g, d.b64, a.lpsi.as<double>(), a.mu.as<double>(),
-                                        a.kv[8].as<double>(), a.sv.as<double>(), a.sg.as<double>(), nullptr, 0,
-                                        d.stream),
+    const ReduceScratch rs{d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>()};
+    HO2D_CUDA(mf_apply_transpose<double>(make_op<double>(d, mesh_, in_.knod, false), a.lpsi.as<double>(),
+                                         a.mu.as<double>(), a.sv.as<double>(), a.sg.as<double>(), a.mu.as<double>(),
+                                         nullptr, nullptr, rs, d.stream),
               "transposed operator");
     launches_ += 2;
     HO2D_CUDA(cudaMemcpyAsync(y, a.mu.get(), nv * 8, cudaMemcpyDeviceToHost, d.stream), "copy");

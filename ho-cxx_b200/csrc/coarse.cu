@@ -281,21 +281,6 @@ unsigned rows_grid(const DevEll<T>& A) {
 
 }  // namespace
 
-// downs, coarsest solve and ups from level 0's right-hand side f0
-template <typename T>
-static void cycle_from(const Precond<T>& pc, const T* f0, const KrylovScalars* sc, cudaStream_t s) {
-    const int d = pc.nlev - 1;
-    for (int l = 0; l < d; ++l) {
-        const CoarseLevel<T>& L = pc.lev[l];
-        k_coarse_rows<T><<<rows_grid(L.M), 256, 0, s>>>(L.M, l ? L.f : f0, DevEll<T>(), nullptr, 0, pc.lev[l + 1].f, sc);
-    }
-    dense_gemv<T>(pc.dense, d ? pc.lev[d].f : f0, pc.lev[d].u, sc, s);
-    for (int l = d - 1; l >= 0; --l) {
-        const CoarseLevel<T>& L = pc.lev[l];
-        k_coarse_rows<T><<<rows_grid(L.S), 256, 0, s>>>(L.S, l ? L.f : f0, L.Q, pc.lev[l + 1].u, 1, L.u, sc);
-    }
-}
-
 template <typename T>
 static bool gemv_forms_f0(const Precond<T>& pc) {
     return pc.nlev == 1 && (size_t)pc.dense.n * sizeof(T) <= kGemvF0Bytes;
@@ -312,24 +297,17 @@ cudaError_t coarse_cycle(const Precond<T>& pc, const BicgVectors<T>& v, const Kr
     }
     const int n0 = pc.lev[0].n;
     k_vertex_rhs<T><<<(unsigned)((n0 + 255) / 256), 256, 0, s>>>(n0, pc.v2e, pc.vw, v, pc.lev[0].f, sc, mode);
-    cycle_from<T>(pc, pc.lev[0].f, sc, s);
-    return cudaGetLastError();
-}
-
-// The whole cycle on a plain level-0 right-hand side f0 (zero-padded to a multiple of 4):
-// u0 = cycle(f0) in pc.lev[0].u. Used by the transposed solve of the adjoint, whose
-// preconditioner forms f0 in its own kernel.
-template <typename T>
-cudaError_t coarse_cycle_vec(const Precond<T>& pc, const T* f0, const KrylovScalars* sc, cudaStream_t s) {
-    if (pc.nlev > 0) cycle_from<T>(pc, f0, sc, s);
-    return cudaGetLastError();
-}
-
-template <typename T>
-int coarse_vec_launches(const Precond<T>& pc) {
-    if (pc.nlev <= 0) return 0;
     const int d = pc.nlev - 1;
-    return d == 0 ? 1 : 2 * d + 1;
+    for (int l = 0; l < d; ++l) {
+        const CoarseLevel<T>& L = pc.lev[l];
+        k_coarse_rows<T><<<rows_grid(L.M), 256, 0, s>>>(L.M, L.f, DevEll<T>(), nullptr, 0, pc.lev[l + 1].f, sc);
+    }
+    dense_gemv<T>(pc.dense, pc.lev[d].f, pc.lev[d].u, sc, s);
+    for (int l = d - 1; l >= 0; --l) {
+        const CoarseLevel<T>& L = pc.lev[l];
+        k_coarse_rows<T><<<rows_grid(L.S), 256, 0, s>>>(L.S, L.f, L.Q, pc.lev[l + 1].u, 1, L.u, sc);
+    }
+    return cudaGetLastError();
 }
 
 template <typename T>
@@ -362,8 +340,6 @@ double coarse_cycle_bytes(const Precond<T>& pc) {
     template cudaError_t coarse_cycle<T>(const Precond<T>&, const BicgVectors<T>&, const KrylovScalars*, int,  \
                                          cudaStream_t);                                                      \
     template int coarse_launches<T>(const Precond<T>&);                                              \
-    template cudaError_t coarse_cycle_vec<T>(const Precond<T>&, const T*, const KrylovScalars*, cudaStream_t); \
-    template int coarse_vec_launches<T>(const Precond<T>&);                                          \
     template double coarse_cycle_bytes<T>(const Precond<T>&);
 
 HO2D_INSTANTIATE_COARSE(double)

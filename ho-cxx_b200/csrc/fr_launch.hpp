@@ -137,6 +137,8 @@ struct MfOp {
     // FP32 operator kernels stage their inputs in shared memory by bulk copies
     // (apply_stage.cuh) instead of reading them through L2 prefetches
     int staged = 0;
+    // the operator is A^T: dinv and h are the transposed ones (the adjoint's solve)
+    int transposed = 0;
     // host side: a second stream and two events; when set, each coarse cycle runs on the
     // second stream beside the fine part of the smoothing step (k_post_a)
     cudaStream_t side = nullptr;
@@ -239,11 +241,6 @@ cudaError_t coarse_cycle(const Precond<T>& pc, const BicgVectors<T>& v, const Kr
                          cudaStream_t s);
 template <typename T>
 int coarse_launches(const Precond<T>& pc);
-// the whole cycle on a plain level-0 right-hand side: u0 -> pc.lev[0].u (coarse.cu)
-template <typename T>
-cudaError_t coarse_cycle_vec(const Precond<T>& pc, const T* f0, const KrylovScalars* sc, cudaStream_t s);
-template <typename T>
-int coarse_vec_launches(const Precond<T>& pc);
 template <typename T>
 double coarse_cycle_bytes(const Precond<T>& pc);
 
@@ -282,6 +279,14 @@ cudaError_t mf_apply_op(const MfOp<T>& op, const T* x, T* xtv, T* xtg, T* y, cud
 // `reps` launches of the operator kernel alone on x whose traces are already in xtv/xtg
 template <typename T>
 cudaError_t mf_apply_only(const MfOp<T>& op, const T* x, const T* xtv, const T* xtg, T* y, int reps, cudaStream_t s);
+// y = A^T x, or with b given r = b - A^T x, ||r||^2 -> sc->rnorm2 and ||b||^2 -> sc->bnorm2; own
+// ([N][K][K]), sv and sg ([N][K][4], boundary entries zero) are scratch; y may be own
+template <typename T>
+cudaError_t mf_apply_transpose(const MfOp<T>& op, const T* x, T* own, T* sv, T* sg, T* y, const T* b, T* r,
+                               const ReduceScratch& rs, cudaStream_t s);
+// the element blocks a ([N][K2][K2], padded_count strides) transposed into at
+template <typename T>
+cudaError_t transpose_blocks(int N, int K, const T* a, T* at, cudaStream_t s);
 int krylov_max_blocks(int K, int N);
 // per-device set-up of the Krylov kernels for order K (krylov.cu): before the first launch
 // or graph capture on the device

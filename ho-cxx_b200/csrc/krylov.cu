@@ -32,6 +32,8 @@
 #include "fr_launch.hpp"
 #include "kron_apply.cuh"
 #include "rows.cuh"
+#include "smoother.cuh"
+#include "rows_transpose.cuh"
 #include "apply_stage.cuh"
 #include "bulk_copy.cuh"
 
@@ -140,7 +142,7 @@ static __host__ __device__ constexpr unsigned rgrid_of(int N) {
 // precision ([K][0] FP64, [K][1] FP32): those kernels loop over element tiles, so one wave
 // covers any mesh and each CTA reduces once. Set by krylov_configure.
 struct WaveSizes {
-    unsigned init = 0, v = 0, t = 0, xr = 0, res = 0, v_st = 0, t_st = 0;
+    unsigned init = 0, v = 0, t = 0, xr = 0, res = 0, v_st = 0, t_st = 0, tr = 0;
 };
 static WaveSizes g_wave[9][2];
 
@@ -226,166 +228,6 @@ __global__ void k_zero_if(T* x, size_t n, const KrylovScalars* sc) {
     if (i < n) x[i] = T(0);
 }
 
-
-// The smoother's element data (BS): 0 = inverse blocks in T; 1 = inverse blocks as BF16 bit
-// patterns (FP32 smoother); 2 = Kronecker-sum factors, with the exact blocks only for the
-// elements the fit does not approximate well (FP32 smoother). Each element's data starts on
-// a 16-byte boundary (padded_count). A warp's EPW blocks (or factor sets) are one
-// contiguous span, copied into shared memory by one bulk copy when the span is at most
-// 26 KB (so a CTA's four spans leave room for two CTAs per SM); larger blocks are read
-// from global memory directly.
-template <int K, typename T, int BS>
-struct PostRows {
-    using DT = typename std::conditional<BS == 1, unsigned short, T>::type;
-    static constexpr int K2 = K * K, K4 = K2 * K2;
-    static constexpr int STRIDE = padded_count(K4, (int)sizeof(DT));  // values of DT per element
-    static constexpr int KF = 4 * K2 + 2 * K;                      // Kronecker factors per element
-    static constexpr int KFS = padded_count(KF, (int)sizeof(T));
-    static constexpr int XSTRIDE = padded_count(K4, (int)sizeof(T));  // compact exact blocks (BS 2)
-    // bytes of one element's staged data: its inverse block, or (BS 2) its factors
-    static constexpr int ELEM = BS == 2 ? KFS * (int)sizeof(T) : STRIDE * (int)sizeof(DT);
-    static constexpr int SPAN = Rows<K>::EPW * ELEM;  // bytes per warp
-    static constexpr bool kStage = SPAN <= 26 * 1024;
-    static constexpr int SMEM = kStage ? Rows<K>::WARPS * SPAN : 0;  // dynamic shared memory
-};
-
-__device__ __forceinline__ float block_value(unsigned short b) { return __uint_as_float((unsigned)b << 16); }
-template <typename T>
-__device__ __forceinline__ T block_value(T v) {
-    return v;
-}
-
-// K consecutive block values (row t of one r-slice of an element block, [rs][ij] layout),
-// widened to T; vector loads as wide as the slice's alignment allows (its offset is a
-// multiple of K values from a 16-byte-aligned block start).
-template <int K, typename T, typename DT>
-__device__ __forceinline__ void load_slice(const DT* p, T (&v)[K]) {
-    constexpr int AL = (K * (int)sizeof(DT)) % 16 == 0 ? 16 : ((K * (int)sizeof(DT)) % 8 == 0 ? 8 : ((K * (int)sizeof(DT)) % 4 == 0 ? 4 : (int)sizeof(DT)));
-    if constexpr (sizeof(DT) == 2) {
-        if constexpr (AL >= 4) {
-#pragma unroll
-            for (int i = 0; i < K; i += 2) {
-                const unsigned w = *reinterpret_cast<const unsigned*>(p + i);
-                v[i] = __uint_as_float(w << 16);
-                v[i + 1] = __uint_as_float(w & 0xffff0000u);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < K; ++i) v[i] = block_value(p[i]);
-        }
-    } else if constexpr (AL == 16 && sizeof(DT) == 4) {
-#pragma unroll
-        for (int i = 0; i < K; i += 4) {
-            const float4 q = *reinterpret_cast<const float4*>(p + i);
-            v[i] = q.x;
-            v[i + 1] = q.y;
-            v[i + 2] = q.z;
-            v[i + 3] = q.w;
-        }
-    } else if constexpr (AL >= 8 && sizeof(DT) == 4) {
-#pragma unroll
-        for (int i = 0; i < K; i += 2) {
-            const float2 q = *reinterpret_cast<const float2*>(p + i);
-            v[i] = q.x;
-            v[i + 1] = q.y;
-        }
-    } else if constexpr (AL == 16 && sizeof(DT) == 8) {
-#pragma unroll
-        for (int i = 0; i < K; i += 2) {
-            const double2 q = *reinterpret_cast<const double2*>(p + i);
-            v[i] = q.x;
-            v[i + 1] = q.y;
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < K; ++i) v[i] = T(p[i]);
-    }
-}
-
-// acc[i] = sum_r blk[r][t K + i] sr[r] over the K^2 values r of the element's residual sr
-// (shared memory): row t of D^-1 sr.
-template <int K, typename T, typename DT>
-__device__ __forceinline__ void block_rows(const DT* blk, const T* sr, int t, T (&acc)[K]) {
-    constexpr int K2 = K * K;
-#pragma unroll
-    for (int i = 0; i < K; ++i) acc[i] = T(0);
-#pragma unroll 4
-    for (int r = 0; r < K2; ++r) {
-        T m[K];
-        load_slice<K, T, DT>(blk + r * K2 + t * K, m);
-        const T s = sr[r];
-#pragma unroll
-        for (int i = 0; i < K; ++i) acc[i] += m[i] * s;
-    }
-}
-
-// The smoother's element inverse M (exact block, BF16 block or Kronecker-sum factors)
-// applied to one element vector held in shared memory (srow, K^2 values, [j][i]): row t of
-// M srow into acc. For BS 2 the transposes are warp-collective, so every lane runs them;
-// zb is a K x K scratch of the element. Warp-collective.
-template <int K, typename T, int BS>
-__device__ __forceinline__ void smoother_rows(const MfOp<T>& op, const typename PostRows<K, T, BS>::DT* blk,
-                                              const T* fk, int kx, const T* srow, T (&zb)[K][K], int t, bool act,
-                                              T (&acc)[K]) {
-    using PS = PostRows<K, T, BS>;
-    constexpr int K2 = K * K;
-    if constexpr (BS == 2) {
-        // exact block where the fit falls back, Kronecker-sum step (fast diagonalisation,
-        // the element body of kron_apply.cuh by rows) for the others
-        const bool kr = act && kx < 0;
-        if (act && kx >= 0) block_rows<K, T, T>(op.kron_exact + (size_t)kx * PS::XSTRIDE, srow, t, acc);
-        const T *vx = fk, *vxi = fk + K2, *vy = fk + 2 * K2, *vyi = fk + 3 * K2, *lx = fk + 4 * K2, *ly = lx + K;
-        T c1[K], r1[K], r2[K], c2[K], c3[K], r3[K];
-        // column t of Vy^-1 R
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            T s = T(0);
-            if (kr) {
-#pragma unroll
-                for (int l = 0; l < K; ++l) s += vyi[j * K + l] * srow[l * K + t];
-            }
-            c1[j] = s;
-        }
-        col_to_row<K, T>(zb, c1, r1, t, kr);
-        // row t of (Vy^-1 R Vx^-T) ./ (ly_t + lx_i)
-#pragma unroll
-        for (int i = 0; i < K; ++i) {
-            T s = T(0);
-            if (kr) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) s += r1[k] * vxi[i * K + k];
-                s = s / (ly[t] + lx[i]);
-            }
-            r2[i] = s;
-        }
-        __syncwarp();  // zb is rewritten next
-        rows_to_col<K, T>(zb, r2, c2, t, kr);
-        // column t of Vy (that), then row t of the product with Vx^T
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            T s = T(0);
-            if (kr) {
-#pragma unroll
-                for (int l = 0; l < K; ++l) s += vy[j * K + l] * c2[l];
-            }
-            c3[j] = s;
-        }
-        __syncwarp();
-        col_to_row<K, T>(zb, c3, r3, t, kr);
-        if (kr) {
-#pragma unroll
-            for (int i = 0; i < K; ++i) {
-                T s = T(0);
-#pragma unroll
-                for (int k = 0; k < K; ++k) s += r3[k] * vx[i * K + k];
-                acc[i] = s;
-            }
-        }
-        __syncwarp();  // zb may be reused by the caller
-    } else {
-        if (act) block_rows<K, T, typename PS::DT>(blk, srow, t, acc);
-    }
-}
 
 // The warp's smoother element data: one bulk copy of its EPW inverse blocks (or factor
 // sets) into its slice of the dynamic shared memory when PostRows::kStage, issued by lane 0
@@ -786,6 +628,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, HatBases<
             // an FP32 solve whose residual has grown a millionfold is lost (krylov_usable
             // then drops its result)
             if (sizeof(T) == 4 && !(out[0] <= 1e12 * sc->bnorm2)) sc->done = 1;
+            if (!isfinite(out[0])) sc->done = 1;
         }
         if (has_handle) cudaGraphSetConditional(h, sc->done ? 0u : 1u);
     }
@@ -846,6 +689,187 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_mf_apply(MfOp<T> op, const
     T yy[K];
     row_apply<K, T>(op, x, xtv, xtg, sm[ix.warp], ix, yy);
     if (ix.active) store_row<K, T>(y + (size_t)ix.el * K * K + ix.t * K, yy);
+}
+
+// ---------------------------------------------------------------- transposed solve
+// BiCGSTAB on A^T mu = b (the discrete adjoint) on the same iteration: the smoother's element
+// inverses and the hats are the transposed ones (op.dinv, op.h), the coarse hierarchy is the
+// forward one (its operator is symmetric), and an operator application is k_tr_own, which
+// also forms the preconditioned vector z = P u0 + w zf, then the gather with its dot products.
+
+// x = 0, r = rhat = b; ||b||^2; element moments of r
+template <int K, typename T>
+__global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_init(int N, HatBases<T> hats, BicgVectors<T> v,
+                                                               ReduceScratch rs) {
+    __shared__ T mom[Rows<K>::WARPS][Rows<K>::EPW][4][K];
+    const int ntiles = (int)rgrid_of<K>(N);
+    double part[1] = {0.0};
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const RowIdx<K> ix(N, tile);
+        T r[K];
+        if (ix.active) {
+            const size_t p = (size_t)ix.el * K * K + ix.t * K;
+            T z[K];
+            load_row<K, T>(v.b + p, r);
+#pragma unroll
+            for (int i = 0; i < K; ++i) {
+                z[i] = T(0);
+                part[0] += double(r[i]) * double(r[i]);
+            }
+            store_row<K, T>(v.x + p, z);
+            store_row<K, T>(v.r + p, r);
+            store_row<K, T>(v.rhat + p, r);
+        }
+        element_moments<K, T>(hats, r, mom[ix.warp][ix.lw], ix, v.er);
+    }
+    double out[1];
+    if (grid_reduce<1>(part, rs.partials, rs.counter, out) && threadIdx.x == 0) {
+        KrylovScalars* sc = rs.sc;
+        sc->rnorm2 = sc->bnorm2 = sc->rho = out[0];
+        sc->eps2 = sc->tol * sc->tol * out[0];
+        sc->rho_old = sc->alpha = sc->omega = 1.0;
+        sc->beta = 0.0;
+        sc->it = 0;
+        sc->breakdown = 0;
+        sc->s_exit = 0;
+        sc->zero_rhs = out[0] == 0.0;
+        sc->done = out[0] == 0.0 || !isfinite(out[0]);
+    }
+}
+
+// z = P u0 + w zf into ph or sh, its own part of A^T z into v or t, and the neighbours' slots.
+// Combining here saves the pass over z that a separate operator launch would read: per point
+// zf read, z and the own part written, three metric coefficients; per face point four
+// coefficients and two slots.
+template <int K, typename T>
+__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 1)
+    k_tr_own(MfOp<T> op, BicgVectors<T> v, const int* __restrict__ conn, const T* __restrict__ u0, double w,
+             const KrylovScalars* sc, int mode) {
+    if (sc->done) return;  // uniform
+    __shared__ RowScratch<K, T> sm[Rows<K>::WARPS];
+    const RowIdx<K> ix(op.g.N, blockIdx.x);
+    const size_t p = (size_t)ix.el * K * K + ix.t * K;
+    T z[K], own[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) z[i] = T(0);
+    if (ix.active) {
+        combine_row<K, T>(op.h, conn, u0, v.zf + p, T(w), ix.el, ix.t, z);
+        store_row<K, T>((mode == 0 ? v.ph : v.sh) + p, z);
+    }
+    row_transpose_own<K, T>(op, z, sm[ix.warp], ix, v.tv, v.tg, own);
+    if (ix.active) store_row<K, T>((mode == 0 ? v.v : v.t) + p, own);
+}
+
+// The gather of v = A^T ph (mode 0: alpha, element moments of v) or t = A^T sh (mode 1: omega),
+// in place over the own part. One wave of CTAs over the element tiles.
+template <int K, typename T>
+__global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_gather(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs,
+                                                                 int mode) {
+    KrylovScalars* sc = rs.sc;
+    if (sc->done || (mode == 1 && sc->s_exit)) return;  // uniform, as in k_mf_v and k_mf_t
+    __shared__ T buf[Rows<K>::WARPS][Rows<K>::EPW][K][K];
+    __shared__ T mom[Rows<K>::WARPS][Rows<K>::EPW][4][K];
+    const int ntiles = (int)rgrid_of<K>(op.g.N);
+    T* y_out = mode == 0 ? v.v : v.t;
+    const T* second = mode == 0 ? v.rhat : v.s;
+    double part[2] = {0.0, 0.0};
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const RowIdx<K> ix(op.g.N, tile);
+        const size_t p = (size_t)ix.el * K * K + ix.t * K;
+        T y[K], q[K];
+        if (ix.active) load_row<K, T>(second + p, q);
+        row_transpose_gather<K, T>(op.b, y_out, v.tv, v.tg, buf[ix.warp][ix.lw], ix, y);
+        if (ix.active) {
+            store_row<K, T>(y_out + p, y);
+#pragma unroll
+            for (int i = 0; i < K; ++i) {
+                part[0] += double(y[i]) * double(q[i]);
+                part[1] += double(y[i]) * double(y[i]);
+            }
+        }
+        if (mode == 0) element_moments<K, T>(op.h, y, mom[ix.warp][ix.lw], ix, v.ev);
+    }
+    double out[2];
+    if (grid_reduce<2>(part, rs.partials, rs.counter, out) && threadIdx.x == 0) {
+        if (mode == 1) {
+            sc->omega = out[1] > 0.0 ? out[0] / out[1] : 0.0;
+        } else if (out[0] == 0.0 || sc->rho == 0.0 || !isfinite(out[0])) {
+            sc->breakdown = 1;
+            sc->done = 1;
+        } else {
+            sc->alpha = sc->rho / out[0];
+        }
+    }
+}
+
+// y = A^T x as the two operator launches alone: own part and slots, then the gather, and with
+// b given r = b - y, ||r||^2 -> rnorm2, ||b||^2 -> bnorm2 (y may then be null).
+template <int K, typename T>
+__global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_apply_own(MfOp<T> op, const T* __restrict__ x,
+                                                                    T* __restrict__ own_out, T* __restrict__ sv,
+                                                                    T* __restrict__ sg) {
+    __shared__ RowScratch<K, T> sm[Rows<K>::WARPS];
+    const RowIdx<K> ix(op.g.N, blockIdx.x);
+    const size_t p = (size_t)ix.el * K * K + ix.t * K;
+    T z[K], own[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) z[i] = T(0);
+    if (ix.active) load_row<K, T>(x + p, z);
+    row_transpose_own<K, T>(op, z, sm[ix.warp], ix, sv, sg, own);
+    if (ix.active) store_row<K, T>(own_out + p, own);
+}
+
+template <int K, typename T>
+__global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_apply_gather(MfOp<T> op, const T* own,
+                                                                       const T* __restrict__ sv,
+                                                                       const T* __restrict__ sg, T* y_out,
+                                                                       const T* __restrict__ b, T* __restrict__ r_out,
+                                                                       ReduceScratch rs) {
+    __shared__ T buf[Rows<K>::WARPS][Rows<K>::EPW][K][K];
+    const int ntiles = (int)rgrid_of<K>(op.g.N);
+    double part[2] = {0.0, 0.0};
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const RowIdx<K> ix(op.g.N, tile);
+        const size_t p = (size_t)ix.el * K * K + ix.t * K;
+        T y[K];
+        row_transpose_gather<K, T>(op.b, own, sv, sg, buf[ix.warp][ix.lw], ix, y);
+        if (!ix.active) continue;
+        if (!b) {
+            store_row<K, T>(y_out + p, y);
+            continue;
+        }
+        T bb[K], r[K];
+        load_row<K, T>(b + p, bb);
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            r[i] = bb[i] - y[i];
+            part[0] += double(r[i]) * double(r[i]);
+            part[1] += double(bb[i]) * double(bb[i]);
+        }
+        store_row<K, T>(r_out + p, r);
+    }
+    if (!b) return;
+    double out[2];
+    if (grid_reduce<2>(part, rs.partials, rs.counter, out) && threadIdx.x == 0) {
+        rs.sc->rnorm2 = out[0];
+        rs.sc->bnorm2 = out[1];
+    }
+}
+
+// The inverse blocks of the transposed operator: D^-T stored as D^-1 is (transposed), so the
+// smoother reads both in the same order. One warp-row per block row; the reads of a warp are
+// contiguous, the writes strided inside one element's few KB.
+template <typename T>
+__global__ void k_transpose_blocks(int N, int K2, int stride, const T* __restrict__ a, T* __restrict__ at) {
+    const size_t n = (size_t)N * K2 * K2, step = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+        const size_t el = i / ((size_t)K2 * K2);
+        const int q = (int)(i - el * K2 * K2), r = q / K2, c = q - r * K2;
+        at[el * stride + (size_t)c * K2 + r] = a[el * stride + q];
+    }
 }
 
 // ---------------------------------------------------------------- FP64 refinement on the device
@@ -951,6 +975,10 @@ template <typename T>
 cudaError_t krylov_init(const MfOp<T>& op, const BicgVectors<T>& v, const ReduceScratch& rs,
                         cudaStream_t s) {
     const int N = op.g.N;
+    if (op.transposed) {
+        HO2D_KSWITCH(op.K, (k_tr_init<KK, T><<<wave_of<KK, T>(&WaveSizes::tr, N), Rows<KK>::THREADS, 0, s>>>(N, op.h, v, rs)));
+        return cudaGetLastError();
+    }
     HO2D_KSWITCH(op.K, (k_trace_in<KK, T><<<rgrid_of<KK>(N), Rows<KK>::THREADS, 0, s>>>(op, v.x, v.xtv, v.xtg)));
     HO2D_KSWITCH(op.K, (k_mf_init<KK, T><<<wave_of<KK, T>(&WaveSizes::init, N), Rows<KK>::THREADS, 0, s>>>(op, v, rs)));
     const size_t n = (size_t)N * op.K * op.K;
@@ -965,8 +993,8 @@ cudaError_t krylov_init(const MfOp<T>& op, const BicgVectors<T>& v, const Reduce
 // set) beside the fine smoothing part k_post_a, then the combination k_post_b. With ev
 // (10 events) everything runs in order on s with the boundaries recorded: ev[0] coarse
 // ev[1] fine part ev[2] combination ev[3] operator ev[4] coarse ev[5] fine part ev[6]
-// combination ev[7] operator ev[8] update ev[9].
-template <int K, typename T>
+// combination ev[7] operator ev[8] update ev[9]. TR: the transposed solve's iteration.
+template <int K, typename T, bool TR = false>
 static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const ReduceScratch& rs, int max_iter,
                            const Precond<T>& pc, cudaGraphConditionalHandle h, int has_handle, cudaStream_t s,
                            cudaEvent_t* ev = nullptr) {
@@ -978,7 +1006,7 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
     const unsigned gp = rgrid_of<K>(N);
     constexpr int tp = Rows<K>::THREADS;
     auto post_a = [&](int mode) {
-        if constexpr (std::is_same<T, float>::value) {
+        if constexpr (std::is_same<T, float>::value && !TR) {
             if (op.kron_f) {
                 k_post_a<K, T, 2><<<gp, tp, PostRows<K, T, 2>::SMEM, s>>>(op, v, mg, rs, mode);
                 return;
@@ -1007,12 +1035,17 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
         post_a(mode);
         if (fork) cudaStreamWaitEvent(s, op.ev_join, 0);
         mark(m0 + 2);
-        k_post_b<K, T><<<gp, tp, 0, s>>>(op, v, mg ? pc.conn : nullptr, pc.lev[0].u, pc.omega, rs.sc, mode);
+        if constexpr (TR) k_tr_own<K, T><<<gp, tp, 0, s>>>(op, v, mg ? pc.conn : nullptr, pc.lev[0].u, pc.omega, rs.sc, mode);
+        else k_post_b<K, T><<<gp, tp, 0, s>>>(op, v, mg ? pc.conn : nullptr, pc.lev[0].u, pc.omega, rs.sc, mode);
     };
     const unsigned gwv = wave_of<K, T>(&WaveSizes::v, N), gwt = wave_of<K, T>(&WaveSizes::t, N),
                    gwx = wave_of<K, T>(&WaveSizes::xr, N);
     // the FP32 operator with its inputs staged by bulk copies, or read through L2 prefetches
     auto apply_v = [&]() {
+        if constexpr (TR) {
+            k_tr_gather<K, T><<<wave_of<K, T>(&WaveSizes::tr, N), tp, 0, s>>>(op, v, rs, 0);
+            return;
+        }
         if constexpr (std::is_same<T, float>::value) {
             if (op.staged) {
                 k_mf_v<K, T, true><<<wave_of<K, T>(&WaveSizes::v_st, N), Rows<K>::THREADS, ApplyStage<K>::CTA_BYTES,
@@ -1023,6 +1056,10 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
         k_mf_v<K, T><<<gwv, Rows<K>::THREADS, 0, s>>>(op, v, rs);
     };
     auto apply_t = [&]() {
+        if constexpr (TR) {
+            k_tr_gather<K, T><<<wave_of<K, T>(&WaveSizes::tr, N), tp, 0, s>>>(op, v, rs, 1);
+            return;
+        }
         if constexpr (std::is_same<T, float>::value) {
             if (op.staged) {
                 k_mf_t<K, T, true><<<wave_of<K, T>(&WaveSizes::t_st, N), Rows<K>::THREADS, ApplyStage<K>::CTA_BYTES,
@@ -1055,6 +1092,7 @@ static cudaError_t configure_waves() {
         out = (unsigned)(nb > 0 ? nb : 1) * (unsigned)sms;
     };
     w(k_xr_update<K, T>, ws.xr);
+    w(k_tr_gather<K, T>, ws.tr);
     if constexpr (sizeof(T) == 4) {  // the FP64 operator kernels take one tile per CTA
         w(k_mf_init<K, T>, ws.init);
         w(k_mf_v<K, T>, ws.v);
@@ -1098,6 +1136,10 @@ int krylov_launches_per_iteration(const Precond<T>& pc) {
 template <typename T>
 cudaError_t krylov_iteration(const MfOp<T>& op, const BicgVectors<T>& v, const ReduceScratch& rs, int max_iter,
                              const Precond<T>& pc, cudaStream_t s) {
+    if (op.transposed) {
+        HO2D_KSWITCH(op.K, (iteration_impl<KK, T, true>(op, v, rs, max_iter, pc, cudaGraphConditionalHandle(), 0, s)));
+        return cudaGetLastError();
+    }
     HO2D_KSWITCH(op.K, (iteration_impl<KK, T>(op, v, rs, max_iter, pc, cudaGraphConditionalHandle(), 0, s)));
     return cudaGetLastError();
 }
@@ -1144,7 +1186,8 @@ cudaError_t krylov_capture_solve(const MfOp<T>& op, const BicgVectors<T>& v, con
     if ((e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
         cudaSuccess)
         return e;
-    HO2D_KSWITCH(op.K, (iteration_impl<KK, T>(op, v, rs, max_iter, pc, h, 1, s)));
+    if (op.transposed) HO2D_KSWITCH(op.K, (iteration_impl<KK, T, true>(op, v, rs, max_iter, pc, h, 1, s)))
+    else HO2D_KSWITCH(op.K, (iteration_impl<KK, T>(op, v, rs, max_iter, pc, h, 1, s)));
     if ((e = cudaStreamEndCapture(s, &body)) != cudaSuccess) return e;
     *graph_out = g;
     return cudaGetLastError();
@@ -1253,6 +1296,21 @@ cudaError_t mf_apply_only(const MfOp<T>& op, const T* x, const T* xtv, const T* 
     return cudaGetLastError();
 }
 
+template <typename T>
+cudaError_t mf_apply_transpose(const MfOp<T>& op, const T* x, T* own, T* sv, T* sg, T* y, const T* b, T* r,
+                               const ReduceScratch& rs, cudaStream_t s) {
+    HO2D_KSWITCH(op.K, (k_tr_apply_own<KK, T><<<rgrid_of<KK>(op.g.N), Rows<KK>::THREADS, 0, s>>>(op, x, own, sv, sg)));
+    HO2D_KSWITCH(op.K, (k_tr_apply_gather<KK, T><<<wave_of<KK, T>(&WaveSizes::tr, op.g.N), Rows<KK>::THREADS, 0, s>>>(
+                           op, own, sv, sg, y, b, r, rs)));
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t transpose_blocks(int N, int K, const T* a, T* at, cudaStream_t s) {
+    k_transpose_blocks<T><<<8 * 148, 256, 0, s>>>(N, K * K, padded_count(K * K * K * K, (int)sizeof(T)), a, at);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_copy_d2f(const double* a, float* b, size_t n, cudaStream_t s) {
     if (n) k_d2f<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, b, n);
     return cudaGetLastError();
@@ -1275,8 +1333,11 @@ cudaError_t launch_axpy_f2d(const float* e, double* x, size_t n, cudaStream_t s)
     template cudaError_t mf_residual<T>(const MfOp<T>&, const double*, const T*, T*, T*, double*,                 \
                                         const ReduceScratch&, cudaStream_t);                                      \
     template cudaError_t mf_apply_op<T>(const MfOp<T>&, const T*, T*, T*, T*, cudaStream_t);                      \
-    template cudaError_t mf_apply_only<T>(const MfOp<T>&, const T*, const T*, const T*, T*, int, cudaStream_t);
+    template cudaError_t mf_apply_only<T>(const MfOp<T>&, const T*, const T*, const T*, T*, int, cudaStream_t);   \
+    template cudaError_t transpose_blocks<T>(int, int, const T*, T*, cudaStream_t);
 
+template cudaError_t mf_apply_transpose<double>(const MfOp<double>&, const double*, double*, double*, double*, double*,
+                                                const double*, double*, const ReduceScratch&, cudaStream_t);
 HO2D_INSTANTIATE_KRYLOV(double)
 HO2D_INSTANTIATE_KRYLOV(float)
 

@@ -145,15 +145,12 @@ struct DeviceState {
 // Device state of the discrete adjoint, allocated on first use.
 struct AdjointState {
     bool ready = false;
-    // preconditioner of the transposed Poisson problem: column sums of A's blocks, and the
-    // coarse hierarchy of (P^T A P)^T
-    std::vector<std::unique_ptr<LevelBufs>> lev;
-    DeviceBuffer dense64, dense32, rowsumT64, rowsumT32;
-    Precond<double> pc64;
-    Precond<float> pc32;
-    // BiCGSTAB on A^T: x r rhat p v s t ph sh dir (sized for FP64), element sums, slots
-    DeviceBuffer kv[10];
-    DeviceBuffer f0, sv, sg, partials, counter, scalars;
+    // the transposed inverse blocks (one copy per precision, made when first used); the rest
+    // of the transposed solve's preconditioner is the forward one's
+    DeviceBuffer dinvT64, dinvT32;
+    // BiCGSTAB on A^T: r rhat p v s t ph sh (sized for FP64), slots [N][K][4]
+    DeviceBuffer kv[8];
+    DeviceBuffer sv, sg;
     DeviceBuffer res64, x32, b32;  // refinement: FP64 residual, FP32 correction and right-hand side
     SolveGraph graph[2];           // captured transposed solves (FP64, FP32) and their operands
     const void* graph_x[2] = {nullptr, nullptr};
