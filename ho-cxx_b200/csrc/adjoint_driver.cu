@@ -112,7 +112,7 @@ Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
     v.tv = a.sv.as<T>();
     v.tg = a.sg.as<T>();
     const Precond<T>& pc = *reinterpret_cast<const Precond<T>*>(f32 ? (const void*)&d.pc32 : (const void*)&d.pc64);
-    const ReduceScratch rs{d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>()};
+    const ReduceScratch rs = reduce_scratch(d);
     // the boundary entries of the slots must read as zero in precision T; the FP64 and FP32
     // solves share these buffers
     HO2D_CUDA(cudaMemsetAsync(a.sv.get(), 0, a.sv.bytes(), d.stream), "memset");
@@ -132,7 +132,7 @@ Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
         SolveGraph& sg = a.graph[gi];
         if (!sg.exec || sg.max_iter != max_iter_ || a.graph_x[gi] != (const void*)x || a.graph_b[gi] != (const void*)b) {
             sg.reset();
-            HO2D_CUDA(krylov_capture_solve<T>(op, v, rs, max_iter_, pc, d.stream, &sg.graph), "graph capture");
+            HO2D_CUDA(krylov_capture_solve<T>(op, v, rs, max_iter_, pc, d.stream, &sg.graph, &sg.one_kernel), "graph capture");
             HO2D_CUDA(cudaGraphInstantiate(&sg.exec, sg.graph, cudaGraphInstantiateFlagUseNodePriority),
                       "graph instantiate");
             sg.max_iter = max_iter_;
@@ -142,7 +142,7 @@ Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
         HO2D_CUDA(cudaGraphLaunch(sg.exec, d.stream), "graph launch");
         HO2D_TRY(poll());
         iters = d.h_sc->it;
-        launches_ += 2 + (int64_t)iters * krylov_launches_per_iteration(pc);
+        launches_ += sg.one_kernel ? 1 : 2 + (int64_t)iters * krylov_launches_per_iteration(pc);
         return {0, ""};
     }
     HO2D_CUDA(krylov_init<T>(op, v, rs, d.stream), "transposed init");
@@ -171,7 +171,7 @@ Error Solver::transposed_solve(const double* rhs, double* mu) {
     AdjointState& a = *adj_;
     const int N = mesh_.n_el, K = in_.knod;
     const size_t nv = (size_t)N * K * K;
-    const ReduceScratch rs{d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>()};
+    const ReduceScratch rs = reduce_scratch(d);
     bool finite = true;
     last_adj_iters_ = 0;
     int sweeps = 0;
@@ -324,7 +324,7 @@ Error Solver::apply_poisson_transpose(const double* x, double* y) {
     HO2D_CUDA(cudaMemcpyAsync(a.lpsi.get(), x, nv * 8, cudaMemcpyHostToDevice, d.stream), "copy");
     HO2D_CUDA(cudaMemsetAsync(a.sv.get(), 0, a.sv.bytes(), d.stream), "memset");  // shared with FP32
     HO2D_CUDA(cudaMemsetAsync(a.sg.get(), 0, a.sg.bytes(), d.stream), "memset");
-    const ReduceScratch rs{d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>()};
+    const ReduceScratch rs = reduce_scratch(d);
     HO2D_CUDA(mf_apply_transpose<double>(make_op<double>(d, mesh_, in_.knod, false), a.lpsi.as<double>(),
                                          a.mu.as<double>(), a.sv.as<double>(), a.sg.as<double>(), a.mu.as<double>(),
                                          nullptr, nullptr, rs, d.stream),

@@ -193,6 +193,8 @@ struct ReduceScratch {
     double* partials;    // [4 * max_blocks]
     unsigned* counter;   // 1 word, zero between launches
     KrylovScalars* sc;   // device scalars
+    double* fused_partials = nullptr;  // FusedScratch of the one-kernel solve
+    unsigned* fused_bar = nullptr;
 };
 
 // Row-padded sparse matrix on the device: row i holds w entries at [i * w, (i + 1) * w);
@@ -257,18 +259,20 @@ int krylov_launches_per_iteration(const Precond<T>& pc);
 template <typename T>
 cudaError_t krylov_iteration_timed(const MfOp<T>& op, const BicgVectors<T>& v, const ReduceScratch& rs, int max_iter,
                                    const Precond<T>& pc, cudaEvent_t* ev, cudaStream_t s);
-// a whole solve (initial residual + device-side while loop of iterations) as a CUDA graph
+// a whole solve (initial residual + device-side while loop of iterations, or for a small mesh one
+// kernel: one_kernel) as a CUDA graph
 template <typename T>
 cudaError_t krylov_capture_solve(const MfOp<T>& op, const BicgVectors<T>& v, const ReduceScratch& rs, int max_iter,
-                                 const Precond<T>& pc, cudaStream_t s, cudaGraph_t* graph_out);
+                                 const Precond<T>& pc, cudaStream_t s, cudaGraph_t* graph_out, bool* one_kernel);
 // a whole mixed-precision solve (FP64 refinement around the FP32 BiCGSTAB, both loops on
 // the device) as a CUDA graph; the refinement controls are read from the scalars
 // (tol_outer, inner_tol, max_sweeps) and its results written there (krylov.cu)
 cudaError_t krylov_capture_refined_solve(const MfOp<double>& A64, const MfOp<float>& A32,
                                          const BicgVectors<float>& v32, const ReduceScratch& rs, int max_iter,
                                          const Precond<float>& pc, double* psi64, const double* rhs, double* r64,
-                                         double* xtv64, double* xtg64, cudaStream_t s, cudaGraph_t* graph_out);
-int krylov_refined_launches(int sweeps, int inner_iters, const Precond<float>& pc);
+                                         double* xtv64, double* xtg64, cudaStream_t s, cudaGraph_t* graph_out,
+                                         bool* one_kernel);
+int krylov_refined_launches(int sweeps, int inner_iters, const Precond<float>& pc, bool one_kernel);
 // r = b - A x with ||r||^2 -> sc->rnorm2, ||b||^2 -> sc->bnorm2 (traces of x into xtv/xtg)
 template <typename T>
 cudaError_t mf_residual(const MfOp<T>& op, const double* b, const T* x, T* xtv, T* xtg, double* r,
@@ -279,6 +283,17 @@ cudaError_t mf_apply_op(const MfOp<T>& op, const T* x, T* xtv, T* xtg, T* y, cud
 // `reps` launches of the operator kernel alone on x whose traces are already in xtv/xtg
 template <typename T>
 cudaError_t mf_apply_only(const MfOp<T>& op, const T* x, const T* xtv, const T* xtg, T* y, int reps, cudaStream_t s);
+// A whole solve as one kernel (krylov_fused.cuh), enqueued on s where the mesh is small enough
+// for it (fits). FusedScratch: 6 kFusedMaxGrid partial sums and the two words of the grid
+// barrier (zero before the first use).
+constexpr int kFusedMaxGrid = 512;
+struct FusedScratch {
+    double* partials = nullptr;
+    unsigned* bar = nullptr;
+};
+template <typename T>
+cudaError_t krylov_fused(const MfOp<T>& op, const BicgVectors<T>& v, const FusedScratch& fs, int max_iter,
+                         const Precond<T>& pc, KrylovScalars* sc, cudaStream_t s, bool* fits);
 // y = A^T x, or with b given r = b - A^T x, ||r||^2 -> sc->rnorm2 and ||b||^2 -> sc->bnorm2; own
 // ([N][K][K]), sv and sg ([N][K][4], boundary entries zero) are scratch; y may be own
 template <typename T>

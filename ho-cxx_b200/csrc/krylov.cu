@@ -1151,20 +1151,54 @@ cudaError_t krylov_iteration_timed(const MfOp<T>& op, const BicgVectors<T>& v, c
     return cudaGetLastError();
 }
 
+// the instances of the one-kernel solve (krylov_fused_*.cu)
+#define HO2D_FUSED_DECL(NAME, T)                                                                               \
+    cudaError_t NAME(const MfOp<T>&, const BicgVectors<T>&, const FusedScratch&, int, const Precond<T>&,        \
+                     KrylovScalars*, cudaStream_t, bool*)
+HO2D_FUSED_DECL(fused_f64, double);
+HO2D_FUSED_DECL(fused_tr64, double);
+HO2D_FUSED_DECL(fused_f32_exact, float);
+HO2D_FUSED_DECL(fused_f32_bf16, float);
+HO2D_FUSED_DECL(fused_f32_kron, float);
+HO2D_FUSED_DECL(fused_tr32, float);
+
+template <typename T>
+cudaError_t krylov_fused(const MfOp<T>& op, const BicgVectors<T>& v, const FusedScratch& fs, int max_iter,
+                         const Precond<T>& pc, KrylovScalars* sc, cudaStream_t s, bool* fits) {
+    if constexpr (std::is_same<T, float>::value) {
+        if (op.transposed) return fused_tr32(op, v, fs, max_iter, pc, sc, s, fits);
+        if (op.kron_f) return fused_f32_kron(op, v, fs, max_iter, pc, sc, s, fits);
+        if (op.dinv_bf16) return fused_f32_bf16(op, v, fs, max_iter, pc, sc, s, fits);
+        return fused_f32_exact(op, v, fs, max_iter, pc, sc, s, fits);
+    } else {
+        if (op.transposed) return fused_tr64(op, v, fs, max_iter, pc, sc, s, fits);
+        return fused_f64(op, v, fs, max_iter, pc, sc, s, fits);
+    }
+}
+
 // Captures a whole solve into `*graph_out`: initial residual, then a while node whose body
 // is one BiCGSTAB iteration; the loop condition lives on the device, so a solve is one
-// graph launch with no host round trip.
+// graph launch with no host round trip. A small mesh's solve is one kernel (krylov_fused).
 template <typename T>
 cudaError_t krylov_capture_solve(const MfOp<T>& op, const BicgVectors<T>& v, const ReduceScratch& rs,
-                                 int max_iter, const Precond<T>& pc, cudaStream_t s, cudaGraph_t* graph_out) {
+                                 int max_iter, const Precond<T>& pc, cudaStream_t s, cudaGraph_t* graph_out,
+                                 bool* one_kernel) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaGraphCreate(&g, 0);
     if (e != cudaSuccess) return e;
-    cudaGraphConditionalHandle h;
-    if ((e = cudaGraphConditionalHandleCreate(&h, g, 0, 0)) != cudaSuccess) return e;
     if ((e = cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
         cudaSuccess)
         return e;
+    bool& fused = *one_kernel;
+    if ((e = krylov_fused<T>(op, v, {rs.fused_partials, rs.fused_bar}, max_iter, pc, rs.sc, s, &fused)) != cudaSuccess)
+        return e;
+    if (fused) {
+        if ((e = cudaStreamEndCapture(s, &g)) != cudaSuccess) return e;
+        *graph_out = g;
+        return cudaGetLastError();
+    }
+    cudaGraphConditionalHandle h;
+    if ((e = cudaGraphConditionalHandleCreate(&h, g, 0, 0)) != cudaSuccess) return e;
     krylov_init<T>(op, v, rs, s);
     k_set_loop<<<1, 1, 0, s>>>(rs.sc, h);
     cudaStreamCaptureStatus st;
@@ -1202,15 +1236,15 @@ cudaError_t krylov_capture_solve(const MfOp<T>& op, const BicgVectors<T>& v, con
 cudaError_t krylov_capture_refined_solve(const MfOp<double>& A64, const MfOp<float>& A32,
                                          const BicgVectors<float>& v32, const ReduceScratch& rs, int max_iter,
                                          const Precond<float>& pc, double* psi64, const double* rhs, double* r64,
-                                         double* xtv64, double* xtg64, cudaStream_t s, cudaGraph_t* graph_out) {
+                                         double* xtv64, double* xtg64, cudaStream_t s, cudaGraph_t* graph_out,
+                                         bool* one_kernel) {
     const size_t n = (size_t)A64.g.N * A64.K * A64.K;
     const unsigned gn = (unsigned)((n + 255) / 256);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaGraphCreate(&g, 0);
     if (e != cudaSuccess) return e;
-    cudaGraphConditionalHandle ho, hi;
+    cudaGraphConditionalHandle ho, hi = 0;
     if ((e = cudaGraphConditionalHandleCreate(&ho, g, 0, 0)) != cudaSuccess) return e;
-    if ((e = cudaGraphConditionalHandleCreate(&hi, g, 0, 0)) != cudaSuccess) return e;
     // adds a while node on handle h after the capture's current dependencies and returns
     // its body graph; the stream's capture continues after the node
     auto add_while = [&](cudaGraphConditionalHandle h, cudaGraph_t* body) -> cudaError_t {
@@ -1248,14 +1282,25 @@ cudaError_t krylov_capture_refined_solve(const MfOp<double>& A64, const MfOp<flo
         cudaSuccess)
         return e;
     k_refine_prep<<<gn, 256, 0, s>>>(r64, const_cast<float*>(v32.b), v32.x, n);
-    krylov_init<float>(A32, v32, rs, s);
-    k_set_loop<<<1, 1, 0, s>>>(rs.sc, hi);
+    bool& fused = *one_kernel;
+    if ((e = krylov_fused<float>(A32, v32, {rs.fused_partials, rs.fused_bar}, max_iter, pc, rs.sc, s, &fused)) !=
+        cudaSuccess)
+        return e;
     cudaGraph_t inner = nullptr;
-    if ((e = add_while(hi, &inner)) != cudaSuccess) return e;
+    if (!fused) {
+        krylov_init<float>(A32, v32, rs, s);
+        if ((e = cudaGraphConditionalHandleCreate(&hi, g, 0, 0)) != cudaSuccess) return e;
+        k_set_loop<<<1, 1, 0, s>>>(rs.sc, hi);
+        if ((e = add_while(hi, &inner)) != cudaSuccess) return e;
+    }
     k_refine_axpy<<<gn, 256, 0, s>>>(v32.x, psi64, n, rs.sc);
     mf_residual<double>(A64, rhs, psi64, xtv64, xtg64, r64, rs, s);
     k_refine_ctl<<<1, 1, 0, s>>>(rs.sc, ho);
     if ((e = cudaStreamEndCapture(s, &outer)) != cudaSuccess) return e;
+    if (fused) {
+        *graph_out = g;
+        return cudaGetLastError();
+    }
     // one BiCGSTAB iteration
     if ((e = cudaStreamBeginCaptureToGraph(s, inner, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal)) !=
         cudaSuccess)
@@ -1268,8 +1313,10 @@ cudaError_t krylov_capture_refined_solve(const MfOp<double>& A64, const MfOp<flo
 
 // kernel launches of one captured refined solve: begin, residual, decision and fix-up, then
 // per sweep right-hand side, initial residual (3), loop set-up, update, residual and
-// decision, plus the inner iterations
-int krylov_refined_launches(int sweeps, int inner_iters, const Precond<float>& pc) {
+// decision, plus the inner iterations (with the one-kernel inner solve: right-hand side, solve,
+// update, residual (2) and decision)
+int krylov_refined_launches(int sweeps, int inner_iters, const Precond<float>& pc, bool one_kernel) {
+    if (one_kernel) return 5 + sweeps * 6;
     return 5 + sweeps * 9 + inner_iters * krylov_launches_per_iteration(pc);
 }
 
@@ -1329,12 +1376,14 @@ cudaError_t launch_axpy_f2d(const float* e, double* x, size_t n, cudaStream_t s)
     template cudaError_t krylov_iteration_timed<T>(const MfOp<T>&, const BicgVectors<T>&, const ReduceScratch&,   \
                                                    int, const Precond<T>&, cudaEvent_t*, cudaStream_t);           \
     template cudaError_t krylov_capture_solve<T>(const MfOp<T>&, const BicgVectors<T>&, const ReduceScratch&,     \
-                                                 int, const Precond<T>&, cudaStream_t, cudaGraph_t*);             \
+                                                 int, const Precond<T>&, cudaStream_t, cudaGraph_t*, bool*);      \
     template cudaError_t mf_residual<T>(const MfOp<T>&, const double*, const T*, T*, T*, double*,                 \
                                         const ReduceScratch&, cudaStream_t);                                      \
     template cudaError_t mf_apply_op<T>(const MfOp<T>&, const T*, T*, T*, T*, cudaStream_t);                      \
     template cudaError_t mf_apply_only<T>(const MfOp<T>&, const T*, const T*, const T*, T*, int, cudaStream_t);   \
-    template cudaError_t transpose_blocks<T>(int, int, const T*, T*, cudaStream_t);
+    template cudaError_t transpose_blocks<T>(int, int, const T*, T*, cudaStream_t);                               \
+    template cudaError_t krylov_fused<T>(const MfOp<T>&, const BicgVectors<T>&, const FusedScratch&, int,          \
+                                         const Precond<T>&, KrylovScalars*, cudaStream_t, bool*);
 
 template cudaError_t mf_apply_transpose<double>(const MfOp<double>&, const double*, double*, double*, double*, double*,
                                                 const double*, double*, const ReduceScratch&, cudaStream_t);

@@ -1,21 +1,30 @@
-// krylov_fused.cu -- a whole BiCGSTAB solve of a small mesh as one kernel (sm_100a).
+// krylov_fused.cuh -- a whole BiCGSTAB solve of a small mesh as one kernel (sm_100a).
 //
 // On a small mesh an iteration of the captured solve (krylov.cu) is a chain of nine to
-// fifteen dependent launches that each work for a microsecond or two: the gaps between them
-// are the solve. Here one resident grid (cooperative launch) keeps the chain inside a kernel,
-// with a grid barrier where a launch boundary was. The phases are those kernels' bodies on the
-// same element tiles, in the same order:
+// fifteen dependent launches that each work for a microsecond or two: launch gaps and the
+// tails of the grid reductions are the solve. Here one resident grid (cooperative launch)
+// keeps the chain inside a kernel, with a grid barrier where a launch boundary was. The
+// phases are those kernels' bodies on the same element tiles, in the same order:
 //   fine smoothing + restriction | coarse levels | z and its traces | operator | update
+// What bounds it is latency: a barrier (about 1.3 us) and one or two L2 round trips a phase,
+// 9 phases an iteration with a dense level 0, 13 with one level below it. An iteration on the
+// 16 x 16 cavity at K = 4 takes 32 us, 43 as launches.
 // A dot product is one partial sum per CTA; after the barrier every CTA adds all of them in
-// the same order, so the scalars are the same bits everywhere and need no broadcast.
+// the same order, so the scalars are the same bits everywhere and need no broadcast. The
+// operator's, the update's and the smoothing's partial sums have buffers of their own
+// (2 x grid doubles each): a CTA that is ahead never writes where another still reads.
 //
 // Memory. What the kernel itself writes is read with ld.cg (L2): another CTA may have written
 // it, and L1 is not coherent. The static data (metrics, tables, factors) keep the read-only
-// path. When every CTA has one tile and the smoother's element data fit, they are copied
-// into shared memory once and stay there for the whole solve.
+// path. Every CTA has at most one tile; its smoother element data are copied into shared
+// memory once and stay there for the whole solve.
 //
 // A barrier's wait is bounded: when it runs out, the CTA records it (dev_error, which the host
 // reports) and returns, and so does every other CTA.
+#pragma once
+
+#include <algorithm>
+
 #include "fr_launch.hpp"
 #include "rows_transpose.cuh"
 #include "smoother.cuh"
@@ -23,6 +32,19 @@
 namespace ho2d {
 
 namespace {
+
+// The line between this kernel and the captured loop of launches, both measured on uniform
+// cavities (ms for 16 solves, loop / one kernel). It pays while every SM has at most one tile:
+// K = 4 FP64 8 tiles 12.9 / 9.4, 113 tiles 16.4 / 14.6, 145 tiles 17.1 / 15.2, 200 tiles
+// 17.4 / 17.6; K = 3 FP64 123 tiles 14.4 / 13.6, 149 tiles 14.4 / 15.0; K = 5 mixed 141 tiles
+// 25.1 / 23.1. At low order the coarse levels outgrow the tiles: K = 2 mixed 4,096 vertices
+// 10.1 / 9.6, 7,921 vertices (127 tiles) 10.2 / 10.8.
+constexpr int kFusedMaxCoarse = 6144;
+// Smallest grid: CTAs without an element tile still work on the coarse levels. 20 solves on the
+// 16 x 16 cavity, K = 4: 66 ms with 8 CTAs, 47.8 with 32, 43.9 with 64, 44.7 with 100, 46.6 with
+// 148; coupled step on 24 x 96 elements 21.0, 20.8, 19.7, 18.7, 18.9 ms.
+constexpr int kFusedMinGrid = 96;
+constexpr int kSmemPerCta = 227 * 1024;
 
 constexpr unsigned kBarrierPolls = 1u << 22;  // about a second of L2 round trips
 
@@ -68,30 +90,25 @@ __device__ __forceinline__ void ldm4(const T* p, T (&v)[4]) {
     ldm_row<4, T>(p, v);
 }
 
-// Grid barrier: bar[0] counts arrivals, bar[1] the barriers passed; both are usable again
-// afterwards without a reset. False: the wait ran out here or in another CTA.
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, int* dev_error, bool& s_ok) {
+// Grid barrier: bar[0] counts arrivals, and barrier number `epoch` of the solve is passed once
+// it reaches base + epoch x grid. (A count that only grows needs one release and one acquire
+// a barrier; resetting it and publishing a generation cost two more L2 round trips, 3 us in
+// all against 1.3.) False: the wait ran out here or in another CTA.
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, int* dev_error, bool& s_ok) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned* gen = bar + 1;
-        const unsigned g = *gen;
-        __threadfence();
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        unsigned n = 0, c;
         bool ok = true;
-        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-            bar[0] = 0u;
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            unsigned n = 0;
-            while (*gen == g) {
-                if (++n > kBarrierPolls) {
-                    atomicExch(dev_error, 1);
-                    ok = false;
-                    break;
-                }
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(bar) : "memory");
+            if ((int)(c - target) >= 0) break;
+            if (++n > kBarrierPolls) {
+                atomicExch(dev_error, 1);
+                ok = false;
+                break;
             }
         }
-        __threadfence();
         s_ok = ok;
     }
     __syncthreads();
@@ -180,7 +197,7 @@ __device__ __forceinline__ void dense_rows(const DevEll<T>& W, const T* f, T* u)
             for (int k = lane; k < W.n; k += 32) acc += T(__uint_as_float((unsigned)__ldg(wr + k) << 16)) * ldm(f + k);
         } else {
             const T* wr = W.val + (size_t)row * W.w;
-#pragma unroll 8
+#pragma unroll 16
             for (int k = lane; k < W.n; k += 32) acc += __ldg(wr + k) * ldm(f + k);
         }
 #pragma unroll
@@ -196,11 +213,12 @@ constexpr int resident_bytes() {
 }
 
 // The solve. BS: the smoother's element data (smoother.cuh); TR: the transposed operator (v.b
-// is the right-hand side and x starts at zero); RES: one tile per CTA, element data resident
-// in shared memory.
-template <int K, typename T, int BS, bool TR, bool RES>
+// is the right-hand side and x starts at zero); One tile per CTA,
+// its element data resident in shared memory.
+template <int K, typename T, int BS, bool TR>
 __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
-    k_fused_solve(MfOp<T> op, BicgVectors<T> v, Precond<T> pc, ReduceScratch rs, unsigned* bar, int max_iter) {
+    k_fused_solve(const __grid_constant__ MfOp<T> op, const __grid_constant__ BicgVectors<T> v,
+                  const __grid_constant__ Precond<T> pc, ReduceScratch rs, unsigned* bar, int max_iter) {
     using R = Rows<K>;
     using PS = PostRows<K, T, BS>;
     using DT = typename PS::DT;
@@ -216,7 +234,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
     const unsigned char* el_data = BS == 2 ? reinterpret_cast<const unsigned char*>(op.kron_f)
                                  : BS == 1 ? reinterpret_cast<const unsigned char*>(op.dinv_bf16)
                                            : reinterpret_cast<const unsigned char*>(op.dinv);
-    if constexpr (RES) {
+    {
         const int e0 = blockIdx.x * R::EPC, ne = max(0, min(R::EPC, N - e0));
         const uint4* src = reinterpret_cast<const uint4*>(el_data + (size_t)e0 * PS::ELEM);
         uint4* dst = reinterpret_cast<uint4*>(res_dyn);
@@ -227,7 +245,9 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
     double rho = 0.0, rho_old = 1.0, alpha = 1.0, omega = 1.0, rnorm2 = 0.0, bnorm2 = 0.0, eps2 = 0.0;
     int it = 0, s_exit = 0, breakdown = 0, zero_rhs = 0;
     bool done = false;
-    auto sync = [&]() { return grid_barrier(bar, &sc->dev_error, s_ok); };
+    // bar[1]: the count at the end of the previous solve, written by its CTA 0
+    unsigned target = __ldcg(bar + 1);
+    auto sync = [&]() { return grid_barrier(bar, target += gridDim.x, &sc->dev_error, s_ok); };
 
     // traces of x, the initial residual's operand
     if constexpr (!TR) {
@@ -337,8 +357,6 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
             mode = 3;
         }
         if (done) break;
-        // (sum_partials' last barrier separates these reads from the next partial sums of this
-        // CTA only: the others' are written after the next grid barrier)
     update:
         if (mode == 3) {  // x, r and the end of the iteration
             double up[2] = {0.0, 0.0};
@@ -437,8 +455,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
                     for (int c = t; c < 4; c += K) v.ep[(it + 1) & 1][el * 4 + c] = moment(el * 4 + c);
             }
             __syncwarp();
-            const size_t eo = (size_t)(ix.active ? el : 0) * PS::ELEM;
-            const unsigned char* data = RES ? res_dyn + (size_t)(ix.warp * R::EPW + ix.lw) * PS::ELEM : el_data + eo;
+            const unsigned char* data = res_dyn + (size_t)(ix.warp * R::EPW + ix.lw) * PS::ELEM;
             int kx = -1;
             if constexpr (BS == 2) {
                 if (ix.active) kx = __ldg(op.kron_x + el);
@@ -461,10 +478,10 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
                 f[r] = acc;
             }
         }
-        if (mode == 1) store_partials<2, NT>(sp, rs.partials, red);
+        if (mode == 1) store_partials<2, NT>(sp, rs.partials + 4 * gridDim.x, red);
         if (!sync()) return;
         if (mode == 1) {
-            sum_partials<2, NT>(rs.partials, out, red);
+            sum_partials<2, NT>(rs.partials + 4 * gridDim.x, out, red);
             if (out[0] <= eps2) {
                 s_exit = 1;
                 rnorm2 = out[0];
@@ -529,6 +546,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
         for (size_t i = (size_t)blockIdx.x * NT + threadIdx.x; i < (size_t)N * K2; i += (size_t)gridDim.x * NT)
             v.x[i] = T(0);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        bar[1] = target;
         sc->rho = rho;
         sc->rho_old = rho_old;
         sc->alpha = alpha;
@@ -543,6 +561,53 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
         sc->done = 1;
     }
 }
+
+// Launches the solve when the mesh fits: a tile for each CTA of the resident grid.
+template <int K, typename T, int BS, bool TR>
+cudaError_t fused_launch(const MfOp<T>& op, const BicgVectors<T>& v, const FusedScratch& fs, int max_iter,
+                         const Precond<T>& pc, KrylovScalars* sc, cudaStream_t s, bool* fits) {
+    *fits = false;
+    constexpr int dyn = resident_bytes<K, T, BS>();
+    if constexpr (dyn + (int)sizeof(RowScratch<K, T>) * Rows<K>::WARPS + 1024 <= kSmemPerCta) {
+        auto kern = k_fused_solve<K, T, BS, TR>;
+        cudaError_t e;
+        int dev = 0, sms = 0, nb = 0;
+        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn)) != cudaSuccess) return e;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, Rows<K>::THREADS, dyn)) != cudaSuccess)
+            return e;
+        const int tiles = (op.g.N + Rows<K>::EPC - 1) / Rows<K>::EPC, cap = std::min(nb * sms, kFusedMaxGrid);
+        if (cap < kFusedMinGrid || tiles > std::min(cap, sms) || (pc.nlev > 0 && pc.lev[0].n > kFusedMaxCoarse))
+            return cudaSuccess;
+        *fits = true;
+        cudaLaunchConfig_t cfg = {};
+        // at least a warp for every row of the dense level, and kFusedMinGrid for the others
+        const int rows = pc.nlev > 0 ? (pc.dense.n + Rows<K>::WARPS - 1) / Rows<K>::WARPS : 0;
+        cfg.gridDim = dim3((unsigned)std::min(cap, std::max(std::max(tiles, rows), kFusedMinGrid)));
+        cfg.blockDim = dim3(Rows<K>::THREADS);
+        cfg.dynamicSmemBytes = dyn;
+        cfg.stream = s;
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        const ReduceScratch rs{fs.partials, nullptr, sc};
+        return cudaLaunchKernelEx(&cfg, kern, op, v, pc, rs, fs.bar, max_iter);
+    }
+    return cudaSuccess;
+}
+
+#define HO2D_FUSED_SWITCH(K, CALL)                         \
+    switch (K) {                                           \
+        case 2: { constexpr int KK = 2; return CALL; }     \
+        case 3: { constexpr int KK = 3; return CALL; }     \
+        case 4: { constexpr int KK = 4; return CALL; }     \
+        case 5: { constexpr int KK = 5; return CALL; }     \
+        case 6: { constexpr int KK = 6; return CALL; }     \
+        default: *fits = false; return cudaSuccess;        \
+    }
 
 }  // namespace
 }  // namespace ho2d

@@ -258,17 +258,13 @@ struct ApplyIn {
     int code[4];
 };
 
-// The operator's inputs from global memory (zeros for an inactive thread).
+// The operator's static inputs (zeros for an inactive thread).
 template <int K, typename T>
-__device__ __forceinline__ void row_apply_load(const PoisGeom<T>& g, const T* __restrict__ x,
-                                               const T* __restrict__ tvin, const T* __restrict__ tgin,
-                                               const RowIdx<K>& ix, ApplyIn<K, T>& in) {
+__device__ __forceinline__ void row_apply_static(const PoisGeom<T>& g, const RowIdx<K>& ix, ApplyIn<K, T>& in) {
     constexpr int K2 = K * K;
     const int t = ix.t, el = ix.el;
     if (ix.active) {
         const size_t e2 = (size_t)el * K2;
-        load_row<K, T>(x + e2 + t * K, in.xr);
-        load_col<K, T>(x + e2 + t, in.xc);
         load_row<K, T>(g.G11 + e2 + t * K, in.g11);
         load_row<K, T>(g.G12 + e2 + t * K, in.g12r);
         load_col<K, T>(g.G22 + e2 + t, in.g22);
@@ -278,18 +274,38 @@ __device__ __forceinline__ void row_apply_load(const PoisGeom<T>& g, const T* __
         load4<T>(g.fb + q4, in.fb);
         load4<T>(g.nfa + q4, in.nfa);
         load4<T>(g.nfb + q4, in.nfb);
-        load4<T>(tvin + q4, in.ntv);
-        load4<T>(tgin + q4, in.ntg);
         load4i(g.code + el * 4, in.code);
     } else {
 #pragma unroll
-        for (int i = 0; i < K; ++i) in.xr[i] = in.xc[i] = in.g11[i] = in.g12r[i] = in.g22[i] = in.g12c[i] = T(0);
+        for (int i = 0; i < K; ++i) in.g11[i] = in.g12r[i] = in.g22[i] = in.g12c[i] = T(0);
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
-            in.fa[f] = in.fb[f] = in.nfa[f] = in.nfb[f] = in.ntv[f] = in.ntg[f] = T(0);
+            in.fa[f] = in.fb[f] = in.nfa[f] = in.nfb[f] = T(0);
             in.code[f] = -1;
         }
     }
+}
+
+// The operator's inputs from global memory (zeros for an inactive thread).
+template <int K, typename T>
+__device__ __forceinline__ void row_apply_load(const PoisGeom<T>& g, const T* __restrict__ x,
+                                               const T* __restrict__ tvin, const T* __restrict__ tgin,
+                                               const RowIdx<K>& ix, ApplyIn<K, T>& in) {
+    constexpr int K2 = K * K;
+    const int t = ix.t, el = ix.el;
+    if (ix.active) {
+        const size_t e2 = (size_t)el * K2, q4 = ((size_t)el * K + t) * 4;
+        load_row<K, T>(x + e2 + t * K, in.xr);
+        load_col<K, T>(x + e2 + t, in.xc);
+        load4<T>(tvin + q4, in.ntv);
+        load4<T>(tgin + q4, in.ntg);
+    } else {
+#pragma unroll
+        for (int i = 0; i < K; ++i) in.xr[i] = in.xc[i] = T(0);
+#pragma unroll
+        for (int f = 0; f < 4; ++f) in.ntv[f] = in.ntg[f] = T(0);
+    }
+    row_apply_static<K, T>(g, ix, in);
 }
 
 // y = A x, rows: the homogeneous-boundary Poisson operator (the method-2 FR Laplacian

@@ -197,19 +197,11 @@ __device__ __forceinline__ void row_transpose_own(const MfOp<T>& op, const T (&z
     __syncwarp();  // the scratch may be rewritten by the caller's next use
 }
 
-// Second half: row t of y = own + transposed traces of the element's incoming slots.
-// Warp-collective.
+// Second half: y (row t of the own part) += the transposed traces of face point t's incoming
+// slots, values v and normal derivatives d. Warp-collective.
 template <int K, typename T>
-__device__ __forceinline__ void row_transpose_gather(const DevBases<T>& b, const T* __restrict__ own,
-                                                     const T* __restrict__ sv, const T* __restrict__ sg,
-                                                     T (&buf)[K][K], const RowIdx<K>& ix, T (&y)[K]) {
-    T v[4] = {T(0), T(0), T(0), T(0)}, d[4] = {T(0), T(0), T(0), T(0)};
-    if (ix.active) {
-        const size_t q4 = ((size_t)ix.el * K + ix.t) * 4;
-        load4<T>(sv + q4, v);
-        load4<T>(sg + q4, d);
-        load_row<K, T>(own + (size_t)ix.el * K * K + ix.t * K, y);
-    }
+__device__ __forceinline__ void transpose_traces(const DevBases<T>& b, const T (&v)[4], const T (&d)[4], T (&buf)[K][K],
+                                                 const RowIdx<K>& ix, T (&y)[K]) {
     T c[K], r[K];
 #pragma unroll
     for (int j = 0; j < K; ++j)
@@ -222,6 +214,20 @@ __device__ __forceinline__ void row_transpose_gather(const DevBases<T>& b, const
                             d[1] * b.sbgb[i * 2 + 1]);
     }
     __syncwarp();  // buf may be rewritten by the caller's next use
+}
+
+// The second half with the own part and the slots from global memory.
+template <int K, typename T>
+__device__ __forceinline__ void row_transpose_gather(const DevBases<T>& b, const T* own, const T* sv, const T* sg,
+                                                     T (&buf)[K][K], const RowIdx<K>& ix, T (&y)[K]) {
+    T v[4] = {T(0), T(0), T(0), T(0)}, d[4] = {T(0), T(0), T(0), T(0)};
+    if (ix.active) {
+        const size_t q4 = ((size_t)ix.el * K + ix.t) * 4;
+        load4<T>(sv + q4, v);
+        load4<T>(sg + q4, d);
+        load_row<K, T>(own + (size_t)ix.el * K * K + ix.t * K, y);
+    }
+    transpose_traces<K, T>(b, v, d, buf, ix, y);
 }
 
 }  // namespace ho2d

@@ -222,6 +222,8 @@ Error Solver::setup_from_mesh() {
     HO2D_CUDA(upload(d.partials, std::vector<double>((size_t)4 * mb, 0.0)), "alloc partials");
     // the grid reductions' counters: one for the groups of 64 CTAs, one per group
     HO2D_CUDA(upload(d.counter, std::vector<unsigned>(2 + mb / 64, 0u)), "alloc counter");
+    HO2D_CUDA(upload(d.fused_partials, std::vector<double>(6 * kFusedMaxGrid, 0.0)), "alloc partials");
+    HO2D_CUDA(upload(d.fused_bar, std::vector<unsigned>(2, 0u)), "alloc barrier");
     HO2D_CUDA(d.scalars.alloc(sizeof(KrylovScalars)), "alloc scalars");
     HO2D_CUDA(cudaMemset(d.scalars.get(), 0, sizeof(KrylovScalars)), "memset");
     time_ = 0.0;
@@ -648,7 +650,7 @@ Error Solver::poisson_solve() {
     DeviceState& d = *d_;
     const int N = mesh_.n_el, K = in_.knod;
     const size_t nv = (size_t)N * K * K;
-    ReduceScratch rs{d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>()};
+    ReduceScratch rs = reduce_scratch(d);
     if (timing_) HO2D_CUDA(cudaEventRecord(d.evp0, d.stream), "event");
     auto poll = [&]() -> Error {
         HO2D_CUDA(cudaMemcpyAsync(d.h_sc, d.scalars.get(), sizeof(KrylovScalars), cudaMemcpyDeviceToHost, d.stream),
@@ -671,7 +673,7 @@ Error Solver::poisson_solve() {
         if (use_graphs_) {
             if (!sg.exec || sg.max_iter != max_iter_) {
                 sg.reset();
-                HO2D_CUDA(krylov_capture_solve(A, v, rs, max_iter_, pc, d.stream, &sg.graph), "graph capture");
+                HO2D_CUDA(krylov_capture_solve(A, v, rs, max_iter_, pc, d.stream, &sg.graph, &sg.one_kernel), "graph capture");
                 // per-node priorities: the coarse cycle's nodes keep their stream's high priority
                 HO2D_CUDA(cudaGraphInstantiate(&sg.exec, sg.graph, cudaGraphInstantiateFlagUseNodePriority),
                           "graph instantiate");
@@ -680,7 +682,7 @@ Error Solver::poisson_solve() {
             HO2D_CUDA(cudaGraphLaunch(sg.exec, d.stream), "graph launch");
             HO2D_TRY(poll());
             iters = d.h_sc->it;
-            launches_ += 4 + (int64_t)iters * krylov_launches_per_iteration(pc);
+            launches_ += sg.one_kernel ? 1 : 4 + (int64_t)iters * krylov_launches_per_iteration(pc);
             return {0, ""};
         }
         HO2D_CUDA(krylov_init(A, v, rs, d.stream), "krylov init");
@@ -736,7 +738,7 @@ Error Solver::poisson_solve() {
             sg.reset();
             HO2D_CUDA(krylov_capture_refined_solve(A64, A32, v, rs, max_iter_, d.pc32, d.psi64.as<double>(),
                                                    d.rhs.as<double>(), d.rres.as<double>(), d.kxtv.as<double>(),
-                                                   d.kxtg.as<double>(), d.stream, &sg.graph),
+                                                   d.kxtg.as<double>(), d.stream, &sg.graph, &sg.one_kernel),
                       "graph capture");
             // per-node priorities: the coarse cycle's nodes keep their stream's high priority
             HO2D_CUDA(cudaGraphInstantiate(&sg.exec, sg.graph, cudaGraphInstantiateFlagUseNodePriority),
@@ -760,7 +762,7 @@ Error Solver::poisson_solve() {
         last_iters_ = d.h_sc->iters_total;
         finite = d.h_sc->finite != 0;
         last_res_ = d.h_sc->res;
-        launches_ += krylov_refined_launches(sweeps, last_iters_, d.pc32);
+        launches_ += krylov_refined_launches(sweeps, last_iters_, d.pc32, sg.one_kernel);
         if (finite && !(last_res_ <= tol_)) {  // stalled or capped: the FP64 solve finishes
             ++fp64_finishes_;
             refined_res = last_res_;
@@ -1169,7 +1171,7 @@ Error Solver::profile_krylov(int reps, double* ms, double* bytes) {
     const size_t nv = (size_t)N * K2;
     for (cudaEvent_t& e : d.prof_ev)
         if (!e) HO2D_CUDA(cudaEventCreate(&e), "cudaEventCreate");
-    ReduceScratch rs{d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>()};
+    ReduceScratch rs = reduce_scratch(d);
     HO2D_CUDA(cudaStreamSynchronize(d.stream), "sync");
     d.h_sc->tol = 0.0;
     HO2D_CUDA(cudaMemcpyAsync(&d.scalars.as<KrylovScalars>()->tol, &d.h_sc->tol, sizeof(double),

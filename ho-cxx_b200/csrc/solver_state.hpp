@@ -42,6 +42,7 @@ struct SolveGraph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int max_iter = -1;
+    bool one_kernel = false;  // the solve is one kernel (krylov_fused), not a loop of launches
     void reset() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -108,6 +109,7 @@ struct DeviceState {
     DeviceBuffer esum[4];  // element moments [N][4] of r, v, p (two alternating buffers)
     DeviceBuffer ktv, ktg, kxtv, kxtg;  // face traces of the Krylov operand and of x
     DeviceBuffer partials, counter, scalars;
+    DeviceBuffer fused_partials, fused_bar;  // FusedScratch of the one-kernel solve
     KrylovScalars* h_sc = nullptr;
     // two-level preconditioner: per coarse level the row-padded cycle operators M, S, Q
     // (FP64 and FP32 values) and the level's f and u (sized for FP64, reused for FP32)
@@ -297,6 +299,11 @@ MfOp<T> make_op(DeviceState& d, const Mesh& m, int K, bool f32) {
     op.ev_fork = d.ev_fork;
     op.ev_join = d.ev_join;
     return op;
+}
+
+inline ReduceScratch reduce_scratch(DeviceState& d) {
+    return {d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>(),
+            d.fused_partials.as<double>(), d.fused_bar.as<unsigned>()};
 }
 
 template <typename T>

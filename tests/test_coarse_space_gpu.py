@@ -45,3 +45,18 @@ def test_streamfunction_matches_oracle(tmp_path, monkeypatch, mesh, knod, dense,
     psi = solve(inp, precision, w0)
     # residual 1e-13 times the conditioning (below 1e4 at these sizes), as the parity tests
     assert np.abs(psi - c.psi).max() <= 1e-9 * np.abs(c.psi).max()
+
+
+# both sides of the line between the one-kernel solve and the loop of launches (148 tiles of 32
+# elements at K = 4): the same solve as host-driven launches (HO2D_GRAPHS=0) agrees, with the
+# last tile full, one element short and one element over
+@pytest.mark.parametrize("precision", [FP64, MIXED_KRYLOV])
+@pytest.mark.parametrize("nr,nt", [(4, 8), (3, 11), (5, 13), (37, 128), (34, 139), (61, 78)])
+def test_one_kernel_solve_and_launches(tmp_path, monkeypatch, nr, nt, precision):
+    inp = meshgen.make_case("cyl%dx%d" % (nr, nt), str(tmp_path), knod=4, steps=1)
+    w0 = np.random.Generator(np.random.PCG64(9)).standard_normal((nr * nt, 4, 4))
+    psi = solve(inp, precision, w0)
+    monkeypatch.setenv("HO2D_GRAPHS", "0")
+    ref = solve(inp, precision, w0)
+    # both at residual 1e-13; the conditioning of a stretched O-grid of this size is below 1e5
+    assert np.abs(psi - ref).max() <= 2e-8 * np.abs(ref).max()
