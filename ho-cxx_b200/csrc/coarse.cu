@@ -295,9 +295,8 @@ cudaError_t coarse_cycle(const Precond<T>& pc, const BicgVectors<T>& v, const Kr
                                                                                mode);
         return cudaGetLastError();
     }
-    const int n0 = pc.lev[0].n;
+    const int n0 = pc.lev[0].n, d = pc.nlev - 1;
     k_vertex_rhs<T><<<(unsigned)((n0 + 255) / 256), 256, 0, s>>>(n0, pc.v2e, pc.vw, v, pc.lev[0].f, sc, mode);
-    const int d = pc.nlev - 1;
     for (int l = 0; l < d; ++l) {
         const CoarseLevel<T>& L = pc.lev[l];
         k_coarse_rows<T><<<rows_grid(L.M), 256, 0, s>>>(L.M, L.f, DevEll<T>(), nullptr, 0, pc.lev[l + 1].f, sc);

@@ -1006,11 +1006,13 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
     const unsigned gp = rgrid_of<K>(N);
     constexpr int tp = Rows<K>::THREADS;
     auto post_a = [&](int mode) {
-        if constexpr (std::is_same<T, float>::value && !TR) {
+        if constexpr (!TR) {
             if (op.kron_f) {
                 k_post_a<K, T, 2><<<gp, tp, PostRows<K, T, 2>::SMEM, s>>>(op, v, mg, rs, mode);
                 return;
             }
+        }
+        if constexpr (std::is_same<T, float>::value && !TR) {
             if (op.dinv_bf16) {
                 k_post_a<K, T, 1><<<gp, tp, PostRows<K, T, 1>::SMEM, s>>>(op, v, mg, rs, mode);
                 return;
@@ -1114,6 +1116,7 @@ static cudaError_t configure_post() {
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     };
     one(k_post_a<K, double, 0>, PostRows<K, double, 0>::SMEM);
+    one(k_post_a<K, double, 2>, PostRows<K, double, 2>::SMEM);
     one(k_post_a<K, float, 0>, PostRows<K, float, 0>::SMEM);
     one(k_post_a<K, float, 1>, PostRows<K, float, 1>::SMEM);
     one(k_post_a<K, float, 2>, PostRows<K, float, 2>::SMEM);
@@ -1156,6 +1159,7 @@ cudaError_t krylov_iteration_timed(const MfOp<T>& op, const BicgVectors<T>& v, c
     cudaError_t NAME(const MfOp<T>&, const BicgVectors<T>&, const FusedScratch&, int, const Precond<T>&,        \
                      KrylovScalars*, cudaStream_t, bool*)
 HO2D_FUSED_DECL(fused_f64, double);
+HO2D_FUSED_DECL(fused_f64_kron, double);
 HO2D_FUSED_DECL(fused_tr64, double);
 HO2D_FUSED_DECL(fused_f32_exact, float);
 HO2D_FUSED_DECL(fused_f32_bf16, float);
@@ -1172,6 +1176,7 @@ cudaError_t krylov_fused(const MfOp<T>& op, const BicgVectors<T>& v, const Fused
         return fused_f32_exact(op, v, fs, max_iter, pc, sc, s, fits);
     } else {
         if (op.transposed) return fused_tr64(op, v, fs, max_iter, pc, sc, s, fits);
+        if (op.kron_f) return fused_f64_kron(op, v, fs, max_iter, pc, sc, s, fits);
         return fused_f64(op, v, fs, max_iter, pc, sc, s, fits);
     }
 }

@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(128) k_assemble(int el0, int n, AsmBases B, As
     auto inv = [&](int nn, Str<double> a) { return asm_invert(nn, a, rk, piv); };
     const int64_t cnt = assemble_element(el, B, tb, m, o, sc, inv);
     if (diag)  // the filtered diagonal block ([ij][rs]) for a host-side fit
-        for (int i = 0; i < K4; ++i) diag[(size_t)el * K4 + i] = sc.Lc[i];
+        for (int i = 0; i < K4; ++i) diag[(size_t)t * K4 + i] = sc.Lc[i];
     asm_invert(K2, sc.Lc, rk, piv);
     double* di = dinv + (size_t)el * dstride;
     for (int ij = 0; ij < K2; ++ij)
@@ -64,32 +64,30 @@ __global__ void __launch_bounds__(128) k_assemble(int el0, int n, AsmBases B, As
 }
 
 // ---------------------------------------------------------------- Kronecker-sum fit
-// One thread per element: the fit of its filtered diagonal block (diag [N][K4]) and its
-// defect ||I - M D||_2 (E: K4 interleaved scratch); the FP32 factors [vx vxi vy vyi lx ly]
-// of a kept fit at el * fstride, zeros and exact[el] = 1 where the exact block stays.
+// One thread per element: the fit of its filtered diagonal block (diag [n][K4], this chunk's) and
+// its defect ||I - M D||_2 (E: K4 interleaved scratch); the factors [vx vxi vy vyi lx ly] of a
+// kept fit at el * stride in FP64 and, when asked for, FP32; zeros, exact[el] = 1 and
+// kx[el] = el where the exact block stays (kx[el] = -1 elsewhere).
 __global__ void __launch_bounds__(128) k_kron_fit(int el0, int n, int K, const double* __restrict__ diag,
-                                                  double* __restrict__ scratch, float* __restrict__ factors,
-                                                  long long fstride, unsigned char* __restrict__ exact) {
+                                                  double* __restrict__ scratch, double* __restrict__ f64,
+                                                  long long s64, float* __restrict__ f32, long long s32,
+                                                  unsigned char* __restrict__ exact, int* __restrict__ kx) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const int el = el0 + t, K2 = K * K, K4 = K2 * K2, per = 4 * K2 + 2 * K;
-    const Str<double> D{const_cast<double*>(diag) + (size_t)el * K4, 1};
+    const Str<double> D{const_cast<double*>(diag) + (size_t)t * K4, 1};
     KronFitHD f;
     const bool ok = kf_fit(K, D, f);
     const double defect = ok ? kf_defect(f, D, Str<double>{scratch + t, n}) : 0.0;
     const bool ex = !ok || !(defect <= kKronDefectMax);
     exact[el] = ex ? 1 : 0;
-    float* fo = factors + (size_t)el * fstride;
-    if (ex) {
-        for (int i = 0; i < per; ++i) fo[i] = 0.f;
-        return;
-    }
+    kx[el] = ex ? el : -1;
     const double* src[4] = {f.vx, f.vxi, f.vy, f.vyi};
-    for (int a = 0; a < 4; ++a)
-        for (int i = 0; i < K2; ++i) fo[a * K2 + i] = (float)src[a][i];
-    for (int i = 0; i < K; ++i) {
-        fo[4 * K2 + i] = (float)f.lx[i];
-        fo[4 * K2 + K + i] = (float)f.ly[i];
+    double* d = f64 + (size_t)el * s64;
+    for (int i = 0; i < per; ++i) {
+        const double v = ex ? 0.0 : i < 4 * K2 ? src[i / K2][i % K2] : i < 4 * K2 + K ? f.lx[i - 4 * K2] : f.ly[i - 4 * K2 - K];
+        d[i] = v;
+        if (f32) f32[(size_t)el * s32 + i] = (float)v;
     }
 }
 
@@ -270,10 +268,11 @@ cudaError_t dense_invert_device(double* a, int n, int w, cudaStream_t s, bool* s
 // Poisson assembly on the device into the solver's buffers: inverse diagonal blocks
 // (dinv64, padded rows), block row sums (rowsum64), column sums (colsum64), the boundary
 // source (bsrc) and the block columns (bcol); the block sums, block columns and entry count
-// come back to op_ for the coarse hierarchy. With kron_fit, the Kronecker-sum fit of every
-// filtered diagonal block runs on the device too: its FP32 factors go to kron_f and the
-// per-element exact-block flags to kron_ on the host.
-Error Solver::assemble_device(bool kron_fit) {
+// come back to op_ for the coarse hierarchy. The Kronecker-sum fit of every filtered diagonal
+// block follows chunk by chunk: its FP64 factors and exact-block indices go to kron64 and
+// kron64_x (the FP64 solve's smoother), and with kron32 the FP32 factors to kron_f and the
+// per-element exact-block flags to kron_ on the host (smoother kind 2).
+Error Solver::assemble_device(bool kron32) {
     DeviceState& d = *d_;
     const int N = mesh_.n_el, K = in_.knod, K2 = K * K, K4 = K2 * K2, neb = mesh_.n_eb;
     op_ = PoissonOperator();
@@ -318,7 +317,6 @@ Error Solver::assemble_device(bool kron_fit) {
     HO2D_CUDA(dbsum.alloc((size_t)N * 5 * sizeof(double)), "alloc block sums");
     HO2D_CUDA(dnnz.alloc(sizeof(unsigned long long)), "alloc");
     HO2D_CUDA(cudaMemsetAsync(dnnz.get(), 0, sizeof(unsigned long long), d.stream), "memset");
-    if (kron_fit) HO2D_CUDA(ddiag.alloc((size_t)N * K4 * sizeof(double)), "alloc diagonal blocks");
     const AsmOut ao{d.bsrc.as<double>(), d.rowsum64.as<double>(), d.colsum64.as<double>(), dbsum.as<double>(), nullptr,
                     d.bcol.as<int>()};
     // chunks of at most ~2 GB of scratch, a multiple of the CTA size
@@ -326,12 +324,29 @@ Error Solver::assemble_device(bool kron_fit) {
     int chunk = (int)std::min<size_t>((size_t)N, std::max<size_t>(128, ((size_t)2 << 30) / per));
     chunk = (chunk + 127) / 128 * 128;
     HO2D_CUDA(scratch.alloc((size_t)chunk * per), "alloc assembly scratch");
+    HO2D_CUDA(ddiag.alloc((size_t)chunk * K4 * sizeof(double)), "alloc diagonal blocks");
+    const int fper = 4 * K2 + 2 * K;
+    const long long s64 = padded_count(fper, 8), s32 = padded_count(fper, 4);
+    DeviceBuffer dex;
+    HO2D_CUDA(dex.alloc((size_t)N), "alloc exact flags");
+    HO2D_CUDA(d.kron64.alloc(((size_t)N * s64 + 1) * sizeof(double)), "alloc Kronecker factors");
+    HO2D_CUDA(cudaMemsetAsync(d.kron64.get(), 0, d.kron64.bytes(), d.stream), "memset");
+    HO2D_CUDA(d.kron64_x.alloc((size_t)N * sizeof(int)), "alloc Kronecker exact-block index");
+    if (kron32) {
+        HO2D_CUDA(d.kron_f.alloc(((size_t)N * s32 + 1) * sizeof(float)), "alloc Kronecker factors");
+        HO2D_CUDA(cudaMemsetAsync(d.kron_f.get(), 0, d.kron_f.bytes(), d.stream), "memset");
+    }
     for (int el0 = 0; el0 < N; el0 += chunk) {
         const int n = std::min(chunk, N - el0);
         k_assemble<<<(n + 127) / 128, 128, 0, d.stream>>>(el0, n, ab, tb, am, ao, d.dinv64.as<double>(), dstride,
-                                                          kron_fit ? ddiag.as<double>() : nullptr,
-                                                          scratch.as<double>(), dnnz.as<unsigned long long>());
+                                                          ddiag.as<double>(), scratch.as<double>(),
+                                                          dnnz.as<unsigned long long>());
         HO2D_CUDA(cudaGetLastError(), "block assembly");
+        k_kron_fit<<<(n + 127) / 128, 128, 0, d.stream>>>(el0, n, K, ddiag.as<double>(), scratch.as<double>(),
+                                                          d.kron64.as<double>(), s64,
+                                                          kron32 ? d.kron_f.as<float>() : nullptr, s32,
+                                                          dex.as<unsigned char>(), d.kron64_x.as<int>());
+        HO2D_CUDA(cudaGetLastError(), "Kronecker-sum fit");
     }
     HO2D_CUDA(cudaStreamSynchronize(d.stream), "block assembly");
     op_.bsum.resize((size_t)N * 5);
@@ -344,27 +359,10 @@ Error Solver::assemble_device(bool kron_fit) {
               "download block columns");
     HO2D_CUDA(cudaMemcpy(&nnz, dnnz.get(), sizeof(nnz), cudaMemcpyDeviceToHost), "download entry count");
     op_.nnz = (int64_t)nnz;
-    if (kron_fit) {
-        const int per = 4 * K2 + 2 * K;
-        const long long fstride = padded_count(per, 4);
-        HO2D_CUDA(d.kron_f.alloc(((size_t)N * fstride + 1) * sizeof(float)), "alloc Kronecker factors");
-        HO2D_CUDA(cudaMemsetAsync(d.kron_f.get(), 0, d.kron_f.bytes(), d.stream), "memset");
-        DeviceBuffer dex, kscr;
-        HO2D_CUDA(dex.alloc((size_t)N), "alloc exact flags");
-        int kchunk = (int)std::min<size_t>((size_t)N, std::max<size_t>(128, ((size_t)2 << 30) / ((size_t)K4 * 8)));
-        kchunk = (kchunk + 127) / 128 * 128;
-        HO2D_CUDA(kscr.alloc((size_t)kchunk * K4 * sizeof(double)), "alloc fit scratch");
-        for (int el0 = 0; el0 < N; el0 += kchunk) {
-            const int n = std::min(kchunk, N - el0);
-            k_kron_fit<<<(n + 127) / 128, 128, 0, d.stream>>>(el0, n, K, ddiag.as<double>(), kscr.as<double>(),
-                                                              d.kron_f.as<float>(), fstride, dex.as<unsigned char>());
-            HO2D_CUDA(cudaGetLastError(), "Kronecker-sum fit");
-        }
+    if (kron32) {
         kron_ = KronSmoother();
         kron_.K = K;
         kron_.exact.resize(N);
-        // (the handle's stream does not synchronise with the legacy stream's copies)
-        HO2D_CUDA(cudaStreamSynchronize(d.stream), "Kronecker-sum fit");
         HO2D_CUDA(cudaMemcpy(kron_.exact.data(), dex.get(), (size_t)N, cudaMemcpyDeviceToHost), "download exact flags");
         kron_on_device_ = true;
     }

@@ -195,8 +195,10 @@ Error Solver::setup_from_mesh() {
     d.vtk.ready = false;  // the VTK node tables follow the mesh
     d.colsum64.reset();
     kron_on_device_ = false;
+    d.kron64.reset();
+    d.kron64_x.reset();
     if (device_setup_) {
-        // kind 2: the Kronecker-sum fit on the device from the assembled diagonal blocks
+        // with the Kronecker-sum fit of the assembled diagonal blocks
         HO2D_TRY(assemble_device(smoother_kind_ == 2));
     } else {
         HO2D_CUDA(upload(d.bsrc, op_.bsrc.empty() ? std::vector<double>{0.0} : op_.bsrc), "upload");

@@ -99,6 +99,9 @@ struct DeviceState {
     // Kronecker-sum smoother for the FP32 solve (HO2D_SMOOTHER_KRON=1): factors, exact-block
     // index per element, compact exact blocks
     DeviceBuffer kron_f, kron_x, kron_exact;
+    // the same for the FP64 solve (device setup): FP64 factors; an element that keeps its exact
+    // block reads it from dinv64
+    DeviceBuffer kron64, kron64_x;
     // matrix-free operator data: G11, G12, G22, fa, fb, nfa, nfb, minv (PoisGeom)
     DeviceBuffer pg64[8], pg32[8], pcode, pscat;
     std::vector<double> pg_host[8];  // kept for the FP32 copies made on demand
@@ -289,10 +292,11 @@ MfOp<T> make_op(DeviceState& d, const Mesh& m, int K, bool f32) {
     op.b = *reinterpret_cast<const DevBases<T>*>(f32 ? (const void*)&d.b32 : (const void*)&d.b64);
     op.dinv = f32 ? (const T*)d.dinv32.get() : (const T*)d.dinv64.get();
     op.dinv_bf16 = f32 ? (const unsigned short*)d.dinv_bf16.get() : nullptr;
-    const bool kron = f32 && d.kron_f.get();
-    op.kron_f = kron ? (const T*)d.kron_f.get() : nullptr;
-    op.kron_x = kron ? d.kron_x.as<int>() : nullptr;
-    op.kron_exact = kron ? (const T*)d.kron_exact.get() : nullptr;
+    const DeviceBuffer &kf = f32 ? d.kron_f : d.kron64, &kx = f32 ? d.kron_x : d.kron64_x;
+    const bool kron = kf.get();
+    op.kron_f = kron ? (const T*)kf.get() : nullptr;
+    op.kron_x = kron ? kx.as<int>() : nullptr;
+    op.kron_exact = !kron ? nullptr : f32 ? (const T*)d.kron_exact.get() : (const T*)d.dinv64.get();
     op.h = *reinterpret_cast<const HatBases<T>*>(f32 ? (const void*)&d.hat32 : (const void*)&d.hat64);
     op.staged = f32 && d.op_staged ? 1 : 0;
     op.side = d.side;
