@@ -532,7 +532,7 @@ def run_ours(args, rank, world, local, phys):
         top = max((k for k in share if k != "coarse_cycle"), key=share.get)
         names = {"smoother": "k_post_a", "smoother_combine": "k_post_b", "operator": "k_mf_v/k_mf_t",
                  "xr_update": "k_xr_update",
-                 "coarse_cycle": "coarse cycle (k_coarse_rows_f0, k_coarse_rows, k_dense_gemv16, k_coarse_up0)"}
+                 "coarse_cycle": "coarse cycle (k_vertex_rhs, k_coarse_rows, k_dense_gemv16)"}
         ms_top, by_top = pm[top]
         achieved = by_top / (ms_top * 1e-3) / 1e9
         tr = measured_traffic(names[top], args.case, knod, f"mixed/{args.smoother}")

@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_trace_in(MfOp<T> op, const
 // every reducing row kernel it runs as one wave of CTAs, each taking element tiles
 // blockIdx.x, blockIdx.x + gridDim.x, ... and reducing once.
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS) k_mf_init(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs) {
+__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf_init(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs) {
     __shared__ RowScratch<K, T> sm[Rows<K>::WARPS];
     const int ntiles = (int)rgrid_of<K>(op.g.N);
     double part[2] = {0.0, 0.0};
@@ -458,9 +458,12 @@ __device__ __forceinline__ void staged_apply_loop(const MfOp<float>& op, const f
 
 // v = A ph; alpha = rho / (rhat, v); element moments of v. ST: the FP32 loop with staged
 // inputs (dynamic shared memory ApplyStage<K>::CTA_BYTES).
-// (FP32: at most 128 registers, four CTAs per SM)
+// (FP32: at most 128 registers, four CTAs per SM. FP64: at most 168, three: without a limit the
+// compiler takes up to 252 and two CTAs are left to hide the loads. 256 x 512 O-grid at K = 6,
+// us per launch: 130 with two CTAs, 116 with three, 146 with four, which spill; K = 7 on 512 x 512
+// elements 325, 303, 397; K = 5 on 14,625 elements 21.9, 20.0, 22.4)
 template <int K, typename T, bool ST = false>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
     k_mf_v(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs) {
     KrylovScalars* sc = rs.sc;
     // the flag is uniform over the grid (only this kernel's last CTA writes it, after every
@@ -512,9 +515,9 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 1)
 }
 
 // t = A sh; omega = (t, s) / (t, t). ST as in k_mf_v.
-// (FP32: at most 128 registers, four CTAs per SM)
+// (registers as k_mf_v)
 template <int K, typename T, bool ST = false>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
     k_mf_t(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs) {
     KrylovScalars* sc = rs.sc;
     if (sc->done || sc->s_exit) return;  // uniform
@@ -640,7 +643,7 @@ __global__ void k_set_loop(const KrylovScalars* sc, cudaGraphConditionalHandle h
 
 // r = b - A x (FP64 refinement residual); ||r||^2 -> rnorm2, ||b||^2 -> bnorm2
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS) k_mf_residual(MfOp<T> op, const double* __restrict__ b,
+__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf_residual(MfOp<T> op, const double* __restrict__ b,
                                                                    const T* __restrict__ x, const T* __restrict__ xtv,
                                                                    const T* __restrict__ xtg, double* __restrict__ r,
                                                                    ReduceScratch rs) {
@@ -681,7 +684,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_mf_residual(MfOp<T> op, co
 
 // y = A x (operator only)
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS) k_mf_apply(MfOp<T> op, const T* __restrict__ x,
+__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf_apply(MfOp<T> op, const T* __restrict__ x,
                                                                 const T* __restrict__ xtv, const T* __restrict__ xtg,
                                                                 T* __restrict__ y) {
     __shared__ RowScratch<K, T> sm[Rows<K>::WARPS];
@@ -743,7 +746,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_init(int N, HatBases<T>
 // zf read, z and the own part written, three metric coefficients; per face point four
 // coefficients and two slots.
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
     k_tr_own(MfOp<T> op, BicgVectors<T> v, const int* __restrict__ conn, const T* __restrict__ u0, double w,
              const KrylovScalars* sc, int mode) {
     if (sc->done) return;  // uniform

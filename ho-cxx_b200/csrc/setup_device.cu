@@ -9,7 +9,7 @@
 // matches the host assembly bit for bit.
 //
 // Coarsest level (the dense solve of src/HO_2D.cpp:3066-3072's AMG hierarchy, here the
-// last level of the P0 / smoothed-aggregation hierarchy): Gauss-Jordan with partial
+// last level of the smoothed-aggregation hierarchy): Gauss-Jordan with partial
 // pivoting, one pivot per step (a one-CTA pivot kernel, then a row-parallel elimination),
 // in place in the row-padded FP64 storage the coarse cycle reads.
 #include <cuda_runtime.h>
@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(128) k_assemble(int el0, int n, AsmBases B, As
 // ---------------------------------------------------------------- Kronecker-sum fit
 // One thread per element: the fit of its filtered diagonal block (diag [n][K4], this chunk's) and
 // its defect ||I - M D||_2 (E: K4 interleaved scratch); the factors [vx vxi vy vyi lx ly] of a
-// kept fit at el * stride in FP64 and, when asked for, FP32; zeros, exact[el] = 1 and
+// kept fit at el * stride in FP64 and FP32, each when asked for; zeros, exact[el] = 1 and
 // kx[el] = el where the exact block stays (kx[el] = -1 elsewhere).
 __global__ void __launch_bounds__(128) k_kron_fit(int el0, int n, int K, const double* __restrict__ diag,
                                                   double* __restrict__ scratch, double* __restrict__ f64,
@@ -81,12 +81,11 @@ __global__ void __launch_bounds__(128) k_kron_fit(int el0, int n, int K, const d
     const double defect = ok ? kf_defect(f, D, Str<double>{scratch + t, n}) : 0.0;
     const bool ex = !ok || !(defect <= kKronDefectMax);
     exact[el] = ex ? 1 : 0;
-    kx[el] = ex ? el : -1;
+    if (kx) kx[el] = ex ? el : -1;
     const double* src[4] = {f.vx, f.vxi, f.vy, f.vyi};
-    double* d = f64 + (size_t)el * s64;
     for (int i = 0; i < per; ++i) {
         const double v = ex ? 0.0 : i < 4 * K2 ? src[i / K2][i % K2] : i < 4 * K2 + K ? f.lx[i - 4 * K2] : f.ly[i - 4 * K2 - K];
-        d[i] = v;
+        if (f64) f64[(size_t)el * s64 + i] = v;
         if (f32) f32[(size_t)el * s32 + i] = (float)v;
     }
 }
@@ -265,12 +264,18 @@ cudaError_t dense_invert_device(double* a, int n, int w, cudaStream_t s, bool* s
     return cudaSuccess;
 }
 
+// Blocks that stay in L2 are read from there as fast, and the fit, a serial chain of about 10 ms
+// in each thread, would be most of a small mesh's setup: the FP64 smoother keeps the exact
+// blocks below kKronMinBytes of them (FP64 solves of 4,096 elements at K = 5, 20 MB: fine
+// smoothing 14.2 us with blocks, 12.0 with factors; 14,625 elements, 73 MB: 26.9 and 16.6).
+constexpr size_t kKronMinBytes = (size_t)48 << 20;
+
 // Poisson assembly on the device into the solver's buffers: inverse diagonal blocks
 // (dinv64, padded rows), block row sums (rowsum64), column sums (colsum64), the boundary
 // source (bsrc) and the block columns (bcol); the block sums, block columns and entry count
 // come back to op_ for the coarse hierarchy. The Kronecker-sum fit of every filtered diagonal
-// block follows chunk by chunk: its FP64 factors and exact-block indices go to kron64 and
-// kron64_x (the FP64 solve's smoother), and with kron32 the FP32 factors to kron_f and the
+// block follows chunk by chunk where it is used: its FP64 factors and exact-block indices go to
+// kron64 and kron64_x (the FP64 solve's smoother), and with kron32 the FP32 factors to kron_f and the
 // per-element exact-block flags to kron_ on the host (smoother kind 2).
 Error Solver::assemble_device(bool kron32) {
     DeviceState& d = *d_;
@@ -324,14 +329,17 @@ Error Solver::assemble_device(bool kron32) {
     int chunk = (int)std::min<size_t>((size_t)N, std::max<size_t>(128, ((size_t)2 << 30) / per));
     chunk = (chunk + 127) / 128 * 128;
     HO2D_CUDA(scratch.alloc((size_t)chunk * per), "alloc assembly scratch");
-    HO2D_CUDA(ddiag.alloc((size_t)chunk * K4 * sizeof(double)), "alloc diagonal blocks");
+    const bool kron64 = (size_t)N * K4 * sizeof(double) >= kKronMinBytes, fit = kron32 || kron64;
+    if (fit) HO2D_CUDA(ddiag.alloc((size_t)chunk * K4 * sizeof(double)), "alloc diagonal blocks");
     const int fper = 4 * K2 + 2 * K;
     const long long s64 = padded_count(fper, 8), s32 = padded_count(fper, 4);
     DeviceBuffer dex;
     HO2D_CUDA(dex.alloc((size_t)N), "alloc exact flags");
-    HO2D_CUDA(d.kron64.alloc(((size_t)N * s64 + 1) * sizeof(double)), "alloc Kronecker factors");
-    HO2D_CUDA(cudaMemsetAsync(d.kron64.get(), 0, d.kron64.bytes(), d.stream), "memset");
-    HO2D_CUDA(d.kron64_x.alloc((size_t)N * sizeof(int)), "alloc Kronecker exact-block index");
+    if (kron64) {
+        HO2D_CUDA(d.kron64.alloc(((size_t)N * s64 + 1) * sizeof(double)), "alloc Kronecker factors");
+        HO2D_CUDA(cudaMemsetAsync(d.kron64.get(), 0, d.kron64.bytes(), d.stream), "memset");
+        HO2D_CUDA(d.kron64_x.alloc((size_t)N * sizeof(int)), "alloc Kronecker exact-block index");
+    }
     if (kron32) {
         HO2D_CUDA(d.kron_f.alloc(((size_t)N * s32 + 1) * sizeof(float)), "alloc Kronecker factors");
         HO2D_CUDA(cudaMemsetAsync(d.kron_f.get(), 0, d.kron_f.bytes(), d.stream), "memset");
@@ -339,13 +347,15 @@ Error Solver::assemble_device(bool kron32) {
     for (int el0 = 0; el0 < N; el0 += chunk) {
         const int n = std::min(chunk, N - el0);
         k_assemble<<<(n + 127) / 128, 128, 0, d.stream>>>(el0, n, ab, tb, am, ao, d.dinv64.as<double>(), dstride,
-                                                          ddiag.as<double>(), scratch.as<double>(),
+                                                          fit ? ddiag.as<double>() : nullptr, scratch.as<double>(),
                                                           dnnz.as<unsigned long long>());
         HO2D_CUDA(cudaGetLastError(), "block assembly");
+        if (!fit) continue;
         k_kron_fit<<<(n + 127) / 128, 128, 0, d.stream>>>(el0, n, K, ddiag.as<double>(), scratch.as<double>(),
-                                                          d.kron64.as<double>(), s64,
+                                                          kron64 ? d.kron64.as<double>() : nullptr, s64,
                                                           kron32 ? d.kron_f.as<float>() : nullptr, s32,
-                                                          dex.as<unsigned char>(), d.kron64_x.as<int>());
+                                                          dex.as<unsigned char>(),
+                                                          kron64 ? d.kron64_x.as<int>() : nullptr);
         HO2D_CUDA(cudaGetLastError(), "Kronecker-sum fit");
     }
     HO2D_CUDA(cudaStreamSynchronize(d.stream), "block assembly");
@@ -359,11 +369,14 @@ Error Solver::assemble_device(bool kron32) {
               "download block columns");
     HO2D_CUDA(cudaMemcpy(&nnz, dnnz.get(), sizeof(nnz), cudaMemcpyDeviceToHost), "download entry count");
     op_.nnz = (int64_t)nnz;
+    std::vector<unsigned char> exact(N, 0);
+    if (fit) HO2D_CUDA(cudaMemcpy(exact.data(), dex.get(), (size_t)N, cudaMemcpyDeviceToHost), "download exact flags");
+    kron64_exact_ = 0;
+    for (unsigned char x : exact) kron64_exact_ += x ? 1 : 0;
     if (kron32) {
         kron_ = KronSmoother();
         kron_.K = K;
-        kron_.exact.resize(N);
-        HO2D_CUDA(cudaMemcpy(kron_.exact.data(), dex.get(), (size_t)N, cudaMemcpyDeviceToHost), "download exact flags");
+        kron_.exact.swap(exact);
         kron_on_device_ = true;
     }
     return {0, ""};

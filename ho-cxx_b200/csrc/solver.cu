@@ -1233,6 +1233,7 @@ Error Solver::profile_krylov(int reps, double* ms, double* bytes) {
         // and v (and p in mode 0: half the launches) read, p or s and M f written
         const double K4 = (double)K2 * K2;
         double blk = K4 * bw;
+        if (!krylov32_ && d.kron64.get()) blk = (4.0 * K2 + 2 * K) * 8 + (double)kron64_exact_ / N * K4 * 8;
         if (krylov32_ && smoother_kind_ == 1) blk = K4 * 2;
         if (krylov32_ && smoother_kind_ == 2) blk = (4.0 * K2 + 2 * K) * 4 + (double)smoother_exact_ / N * K4 * 4;
         bytes[0] = (double)N * (blk + 4.5 * K2 * bw);

@@ -164,7 +164,7 @@ class Solver {
     Error update_bcs(double t, bool into_stage);
     Error setup_from_mesh();
     Error assemble_device(bool kron_fit);  // setup_device.cu
-    Error ensure_host_colsum();  // block column sums on the host (the adjoint's coarse problem)
+    Error ensure_host_colsum();  // block column sums on the host (get_poisson_setup)
     Error hybrid_upload();
     Error upload_precision_arrays();
     Error setup_preconditioner();
@@ -206,6 +206,7 @@ class Solver {
     int smoother_exact_ = 0;                  // kind 2: elements that keep their exact block
     int device_setup_req_ = -1;               // requested setup place (-1: environment)
     bool device_setup_ = true;                // Poisson assembly on the device since the last setup
+    int kron64_exact_ = 0;                    // FP64 smoother: elements that keep their exact block
     bool kron_on_device_ = false;             // the Kronecker-sum factors were fitted on the device
     // initial guess of each stage's Poisson solve: 0/1 = the last psi; 2, 3 = the same RK
     // stage of the last 2 or 3 steps extrapolated in time (HO2D_PSI_EXTRAP)
