@@ -10,7 +10,7 @@ slowest rank's device time.
 The headline precision is HO2D_MIXED: the FR stage kernels in FP32 (velocity from the FP64
 streamfunction, RK accumulation in FP64) and FP32 BiCGSTAB with the FP32 preconditioner
 inside FP64 iterative refinement of the Poisson solve (the device-resident refinement
-loop). The FP64 plain path (every array and operation in FP64, exact FP64 inverse blocks)
+loop). The FP64 plain path (every array and operation in FP64, FP64 Kronecker-sum factors)
 is timed on the same workload under "fp64", and HO2D_MIXED_KRYLOV (FP64 FR stage, the same
 mixed Poisson solve) under "mixed_fp64_stage", each with its relative L2 vorticity
 difference from FP64 after the same steps and after --l2-steps steps.

@@ -40,7 +40,8 @@ enum ho2d_precision {
 
 /* Smoother of the FP32 Poisson preconditioner (HO2D_MIXED, HO2D_MIXED_KRYLOV). No
  * counterpart in the reference, whose AMGCL relaxation is fixed at compile time
- * (src/HO_2D.hpp:54). The FP64 solve always uses exact FP64 inverse blocks. */
+ * (src/HO_2D.hpp:54). The FP64 solve's smoother is FP64 whatever the
+ * kind: Kronecker-sum factors on large meshes, exact inverse blocks on others. */
 enum ho2d_smoother {
     HO2D_SMOOTHER_BLOCKS = 0,  /* exact inverse of each element's diagonal block, FP32 */
     HO2D_SMOOTHER_BF16 = 1,    /* the same blocks stored in BF16 (half the bytes) */
