@@ -105,8 +105,8 @@ Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
     op.kron_f = op.kron_exact = nullptr;
     op.kron_x = nullptr;
     op.staged = 0;
-    std::swap(op.h.hp, op.h.hr);
     BicgVectors<T> v = krylov_vectors<T>(d, x, b);
+    std::swap(v.h.hp, v.h.hr);
     T** kv[8] = {&v.r, &v.rhat, &v.p, &v.v, &v.s, &v.t, &v.ph, &v.sh};
     for (int i = 0; i < 8; ++i) *kv[i] = a.kv[i].as<T>();
     v.tv = a.sv.as<T>();

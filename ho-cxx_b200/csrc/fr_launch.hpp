@@ -126,7 +126,6 @@ struct MfOp {
     PoisGeom<T> g;
     DevBases<T> b;
     const T* dinv;          // [N][K2][K2] inverse diagonal blocks, transposed ([rs][ij])
-    HatBases<T> h;
     // optional BF16 copy of dinv (bit patterns), read by the FP32 smoother when present
     const unsigned short* dinv_bf16 = nullptr;
     // optional Kronecker-sum smoother (FP32): factors [N][4K^2 + 2K], the compact index of
@@ -137,7 +136,7 @@ struct MfOp {
     // FP32 operator kernels stage their inputs in shared memory by bulk copies
     // (apply_stage.cuh) instead of reading them through L2 prefetches
     int staged = 0;
-    // the operator is A^T: dinv and h are the transposed ones (the adjoint's solve)
+    // the operator is A^T: dinv and the vectors' hats are the transposed ones (the adjoint's solve)
     int transposed = 0;
     // host side: a second stream and two events; when set, each coarse cycle runs on the
     // second stream beside the fine part of the smoothing step (k_post_a)
@@ -156,6 +155,7 @@ struct BicgVectors {
     // and s are linear combinations of them, formed where they are read
     T *er, *ev, *ep[2];
     T* zf;  // the fine part M f of the current preconditioner application (k_post_a)
+    HatBases<T> h;
 };
 
 // The element moments of one preconditioner application's operand, formed where they are

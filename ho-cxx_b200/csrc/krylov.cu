@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf
             store_row<K, T>(v.r + p, r);
             store_row<K, T>(v.rhat + p, r);
         }
-        element_moments<K, T>(op.h, r, sm[ix.warp].com[ix.lw], ix, v.er);
+        element_moments<K, T>(v.h, r, sm[ix.warp].com[ix.lw], ix, v.er);
     };
     // FP32: one wave of CTAs over the tiles; FP64 keeps one tile per CTA (the loop would
     // push the operator past the register file)
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_post_b(MfOp<T> op, BicgVec
     int dst[4];
     if (ix.active) {
         load4i(op.g.scat + ((size_t)ix.el * K + ix.t) * 4, dst);
-        combine_row<K, T>(op.h, conn, u0, v.zf + p, T(w), ix.el, ix.t, zz);
+        combine_row<K, T>(v.h, conn, u0, v.zf + p, T(w), ix.el, ix.t, zz);
         store_row<K, T>((mode == 0 ? v.ph : v.sh) + p, zz);
     }
     row_emit_traces<K, T>(op.b, zb[ix.warp][ix.lw], zz, dst, v.tv, v.tg, ix.t, ix.active);
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
 #pragma unroll
             for (int i = 0; i < K; ++i) part[0] += double(rh[i]) * double(y[i]);
         }
-        element_moments<K, T>(op.h, y, sm[ix.warp].com[ix.lw], ix, v.ev);
+        element_moments<K, T>(v.h, y, sm[ix.warp].com[ix.lw], ix, v.ev);
     };
     auto tile_body = [&](int tile) {
         const RowIdx<K> ix(op.g.N, tile);
@@ -571,8 +571,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
 // max_iter) or finds `done` set and clears the condition, so the device loop always ends.
 // Each thread updates element rows.
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, HatBases<T> hats, BicgVectors<T> v,
-                                                                 ReduceScratch rs, int max_iter,
+__global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, BicgVectors<T> v, ReduceScratch rs, int max_iter,
                                                                  cudaGraphConditionalHandle h, int has_handle) {
     __shared__ T mom[Rows<K>::WARPS][Rows<K>::EPW][4][K];
     KrylovScalars* sc = rs.sc;
@@ -615,7 +614,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_xr_update(int N, HatBases<
                 store_row<K, T>(v.r + p, r);
             }
         }
-        if (!s_exit) element_moments<K, T>(hats, r, mom[ix.warp][ix.lw], ix, v.er);
+        if (!s_exit) element_moments<K, T>(v.h, r, mom[ix.warp][ix.lw], ix, v.er);
     }
     double out[2];
     if (grid_reduce<2>(part, rs.partials, rs.counter, out) && threadIdx.x == 0) {
@@ -696,14 +695,13 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf
 
 // ---------------------------------------------------------------- transposed solve
 // BiCGSTAB on A^T mu = b (the discrete adjoint) on the same iteration: the smoother's element
-// inverses and the hats are the transposed ones (op.dinv, op.h), the coarse hierarchy is the
+// inverses and the hats are the transposed ones (op.dinv, v.h), the coarse hierarchy is the
 // forward one (its operator is symmetric), and an operator application is k_tr_own, which
 // also forms the preconditioned vector z = P u0 + w zf, then the gather with its dot products.
 
 // x = 0, r = rhat = b; ||b||^2; element moments of r
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_init(int N, HatBases<T> hats, BicgVectors<T> v,
-                                                               ReduceScratch rs) {
+__global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_init(int N, BicgVectors<T> v, ReduceScratch rs) {
     __shared__ T mom[Rows<K>::WARPS][Rows<K>::EPW][4][K];
     const int ntiles = (int)rgrid_of<K>(N);
     double part[1] = {0.0};
@@ -724,7 +722,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_init(int N, HatBases<T>
             store_row<K, T>(v.r + p, r);
             store_row<K, T>(v.rhat + p, r);
         }
-        element_moments<K, T>(hats, r, mom[ix.warp][ix.lw], ix, v.er);
+        element_moments<K, T>(v.h, r, mom[ix.warp][ix.lw], ix, v.er);
     }
     double out[1];
     if (grid_reduce<1>(part, rs.partials, rs.counter, out) && threadIdx.x == 0) {
@@ -757,7 +755,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
 #pragma unroll
     for (int i = 0; i < K; ++i) z[i] = T(0);
     if (ix.active) {
-        combine_row<K, T>(op.h, conn, u0, v.zf + p, T(w), ix.el, ix.t, z);
+        combine_row<K, T>(v.h, conn, u0, v.zf + p, T(w), ix.el, ix.t, z);
         store_row<K, T>((mode == 0 ? v.ph : v.sh) + p, z);
     }
     row_transpose_own<K, T>(op, z, sm[ix.warp], ix, v.tv, v.tg, own);
@@ -792,7 +790,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_tr_gather(MfOp<T> op, Bicg
                 part[1] += double(y[i]) * double(y[i]);
             }
         }
-        if (mode == 0) element_moments<K, T>(op.h, y, mom[ix.warp][ix.lw], ix, v.ev);
+        if (mode == 0) element_moments<K, T>(v.h, y, mom[ix.warp][ix.lw], ix, v.ev);
     }
     double out[2];
     if (grid_reduce<2>(part, rs.partials, rs.counter, out) && threadIdx.x == 0) {
@@ -979,7 +977,7 @@ cudaError_t krylov_init(const MfOp<T>& op, const BicgVectors<T>& v, const Reduce
                         cudaStream_t s) {
     const int N = op.g.N;
     if (op.transposed) {
-        HO2D_KSWITCH(op.K, (k_tr_init<KK, T><<<wave_of<KK, T>(&WaveSizes::tr, N), Rows<KK>::THREADS, 0, s>>>(N, op.h, v, rs)));
+        HO2D_KSWITCH(op.K, (k_tr_init<KK, T><<<wave_of<KK, T>(&WaveSizes::tr, N), Rows<KK>::THREADS, 0, s>>>(N, v, rs)));
         return cudaGetLastError();
     }
     HO2D_KSWITCH(op.K, (k_trace_in<KK, T><<<rgrid_of<KK>(N), Rows<KK>::THREADS, 0, s>>>(op, v.x, v.xtv, v.xtg)));
@@ -1081,7 +1079,7 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
     mark(7);
     apply_t();
     mark(8);
-    k_xr_update<K, T><<<gwx, Rows<K>::THREADS, 0, s>>>(N, op.h, v, rs, max_iter, h, has_handle);
+    k_xr_update<K, T><<<gwx, Rows<K>::THREADS, 0, s>>>(N, v, rs, max_iter, h, has_handle);
     mark(9);
 }
 

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
                     }
                 }
             }
-            if (mode != 1) element_moments<K, T>(op.h, y, sm[ix.warp].com[ix.lw], ix, mode == 2 ? v.er : v.ev);
+            if (mode != 1) element_moments<K, T>(v.h, y, sm[ix.warp].com[ix.lw], ix, mode == 2 ? v.er : v.ev);
         }
         store_partials<2, NT>(part, rs.partials, red);
         if (!sync()) return;
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
                     }
                     store_row<K, T>(v.x + p, x);
                 }
-                if (!s_exit) element_moments<K, T>(op.h, r, sm[ix.warp].com[ix.lw], ix, v.er);
+                if (!s_exit) element_moments<K, T>(v.h, r, sm[ix.warp].com[ix.lw], ix, v.er);
             }
             it += 1;
             if (s_exit) break;  // rnorm2 is already ||s||^2
@@ -521,13 +521,13 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
                     T u[4];
 #pragma unroll
                     for (int k = 0; k < 4; ++k) u[k] = c[k] >= 0 ? ldm(pc.lev[0].u + c[k]) : T(0);
-                    const T y0 = op.h.hp[t * 2 + 0], y1 = op.h.hp[t * 2 + 1];
+                    const T y0 = v.h.hp[t * 2 + 0], y1 = v.h.hp[t * 2 + 1];
                     l = u[0] * y0 + u[3] * y1;
                     r = u[1] * y0 + u[2] * y1;
                 }
 #pragma unroll
                 for (int i = 0; i < K; ++i)
-                    z[i] = (l * op.h.hp[i * 2 + 0] + r * op.h.hp[i * 2 + 1]) + T(pc.omega) * f[i];
+                    z[i] = (l * v.h.hp[i * 2 + 0] + r * v.h.hp[i * 2 + 1]) + T(pc.omega) * f[i];
                 store_row<K, T>((mode == 0 ? v.ph : v.sh) + p, z);
             }
             if constexpr (TR) {

@@ -297,7 +297,6 @@ MfOp<T> make_op(DeviceState& d, const Mesh& m, int K, bool f32) {
     op.kron_f = kron ? (const T*)kf.get() : nullptr;
     op.kron_x = kron ? kx.as<int>() : nullptr;
     op.kron_exact = !kron ? nullptr : f32 ? (const T*)d.kron_exact.get() : (const T*)d.dinv64.get();
-    op.h = *reinterpret_cast<const HatBases<T>*>(f32 ? (const void*)&d.hat32 : (const void*)&d.hat64);
     op.staged = f32 && d.op_staged ? 1 : 0;
     op.side = d.side;
     op.ev_fork = d.ev_fork;
@@ -332,6 +331,7 @@ BicgVectors<T> krylov_vectors(DeviceState& d, T* x, const T* b) {
     v.ep[0] = d.esum[2].as<T>();
     v.ep[1] = d.esum[3].as<T>();
     v.zf = d.zf.as<T>();
+    v.h = *reinterpret_cast<const HatBases<T>*>(sizeof(T) == 4 ? (const void*)&d.hat32 : (const void*)&d.hat64);
     return v;
 }
 
