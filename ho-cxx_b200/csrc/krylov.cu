@@ -158,6 +158,7 @@ static unsigned wave_of(unsigned WaveSizes::*which, int N) {
 template <int K, typename T>
 __global__ void __launch_bounds__(Rows<K>::THREADS) k_trace_in(MfOp<T> op, const T* __restrict__ x, T* __restrict__ tv,
                                                                 T* __restrict__ tg) {
+    asm volatile("griddepcontrol.launch_dependents;");  // (k_mf_apply, where it follows)
     __shared__ T buf[Rows<K>::WARPS][Rows<K>::EPW][K][K];
     const RowIdx<K> ix(op.g.N, blockIdx.x);
     T row[K];
@@ -681,16 +682,33 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf
     }
 }
 
-// y = A x (operator only)
+// y = A x (operator only). The traces come from k_trace_in, launched right before it as its
+// programmatic primary (mf_apply_op): everything else is loaded while that kernel still runs,
+// and the traces (read through L2, since they are being written) after it has ended. A call
+// on 9,216 elements at K = 5 is bound by the two launches and the host's synchronisation.
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf_apply(MfOp<T> op, const T* __restrict__ x,
-                                                                const T* __restrict__ xtv, const T* __restrict__ xtg,
-                                                                T* __restrict__ y) {
+__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3)
+    k_mf_apply(MfOp<T> op, const T* __restrict__ x, const T* xtv, const T* xtg, T* __restrict__ y) {
     __shared__ RowScratch<K, T> sm[Rows<K>::WARPS];
     const RowIdx<K> ix(op.g.N, blockIdx.x);
+    const size_t p = (size_t)ix.el * K * K + ix.t * K, q4 = ((size_t)ix.el * K + ix.t) * 4;
+    ApplyIn<K, T> in;
+    row_apply_static<K, T>(op.g, ix, in);
+#pragma unroll
+    for (int i = 0; i < K; ++i) in.xr[i] = in.xc[i] = T(0);
+    if (ix.active) {
+        load_row<K, T>(x + p, in.xr);
+        load_col<K, T>(x + (size_t)ix.el * K * K + ix.t, in.xc);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // returns at once without a primary
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+        in.ntv[f] = ix.active ? __ldcg(xtv + q4 + f) : T(0);
+        in.ntg[f] = ix.active ? __ldcg(xtg + q4 + f) : T(0);
+    }
     T yy[K];
-    row_apply<K, T>(op, x, xtv, xtg, sm[ix.warp], ix, yy);
-    if (ix.active) store_row<K, T>(y + (size_t)ix.el * K * K + ix.t * K, yy);
+    row_apply_core<K, T>(op, in, sm[ix.warp], ix, yy);
+    if (ix.active) store_row<K, T>(y + p, yy);
 }
 
 // ---------------------------------------------------------------- transposed solve
@@ -1338,8 +1356,18 @@ cudaError_t mf_residual(const MfOp<T>& op, const double* b, const T* x, T* xtv, 
 template <typename T>
 cudaError_t mf_apply_op(const MfOp<T>& op, const T* x, T* xtv, T* xtg, T* y, cudaStream_t s) {
     HO2D_KSWITCH(op.K, (k_trace_in<KK, T><<<rgrid_of<KK>(op.g.N), Rows<KK>::THREADS, 0, s>>>(op, x, xtv, xtg)));
-    HO2D_KSWITCH(op.K, (k_mf_apply<KK, T><<<rgrid_of<KK>(op.g.N), Rows<KK>::THREADS, 0, s>>>(op, x, xtv, xtg, y)));
-    return cudaGetLastError();
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    HO2D_KSWITCH(op.K, (cfg.gridDim = dim3(rgrid_of<KK>(op.g.N)), cfg.blockDim = dim3(Rows<KK>::THREADS),
+                        e = cudaLaunchKernelEx(&cfg, k_mf_apply<KK, T>, op, x, (const T*)xtv, (const T*)xtg, y)));
+    return e;
 }
 
 template <typename T>
