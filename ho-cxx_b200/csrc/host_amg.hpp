@@ -42,6 +42,13 @@ struct Ell {
 };
 Ell to_ell(const Csr& A);
 
+// Whether the FP32 preconditioner holds the coarsest inverse in BF16 (half the bytes of the
+// largest coarse read; the preconditioner's precision changes only the iteration count): where
+// it is a level below level 0, on meshes of more than kDense16Elements elements. Smaller ones
+// keep FP32: their coarsest level has a few hundred rows and is read from L2.
+constexpr int kDense16Elements = 1024;
+inline bool dense_in_bf16(int n_el, int levels) { return levels > 1 && n_el > kDense16Elements; }
+
 struct CoarseHierarchy {
     std::vector<AmgLevel> levels;  // levels[0] is the coarse space's own operator
     int n_dense = 0;

@@ -456,10 +456,7 @@ Error Solver::upload_hierarchy(const CoarseHierarchy& H, double omega, std::vect
         HO2D_CUDA(dense_invert_device(dense64.as<double>(), nd, wd, d_->stream, &singular), "dense inverse");
         if (singular) return {3, "singular coarsest Poisson operator"};
     }
-    // the FP32 preconditioner's coarsest inverse in BF16 (half the bytes of the largest
-    // coarse read; the preconditioner's precision changes only the iteration count) when
-    // it is a level below the element level
-    const bool dense16 = nl > 1;
+    const bool dense16 = dense_in_bf16(mesh_.n_el, nl);
     const int w16 = (nd + 7) / 8 * 8;
     if (dense16) {
         HO2D_CUDA(dense32.alloc(((size_t)nd * w16 + 8) * sizeof(uint16_t)), "alloc dense");
