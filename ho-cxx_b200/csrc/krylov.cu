@@ -138,6 +138,24 @@ static __host__ __device__ constexpr unsigned rgrid_of(int N) {
     return (unsigned)((N + Rows<K>::EPC - 1) / Rows<K>::EPC);
 }
 
+// Resident CTAs an SM that the operator kernels' registers are cut down to. In the iteration
+// (k_mf_v, k_mf_t) FP32 takes four (128 registers). FP64 takes three (168) up to order 7: without a
+// limit the compiler takes 162 to 252, and two CTAs are left to hide the loads; at orders 6 and 7
+// three spill 140 to 230 bytes and still win. Order 8 would spill 320 and 410 bytes and keeps its
+// 238 registers. us per launch of k_mf_v / k_mf_t in FP64 with two CTAs and with three: K = 3 on
+// 400 x 400 elements 61.8 / 46.7 and 49.1 / 36.4, K = 4 (340^2) 67.9 / 53.3 and 55.8 / 42.7, K = 5
+// (320^2) 80.4 / 65.2 and 63.8 / 51.4, K = 6 (256^2) 67.0 / 57.3 and 63.3 / 49.5, K = 7 (224^2)
+// 70.0 / 60.0 and 66.0 / 59.5, K = 8 (200^2) 69.4 / 65.8 and 73.3 / 75.9. (Four CTAs spill
+// everywhere: K = 6 on 256 x 512 elements 146 against 116.)
+template <int K, typename T>
+constexpr int kOperatorCtas = sizeof(T) == 4 ? 4 : (K <= 7 ? 3 : 1);
+// The residuals (k_mf_init, k_mf_residual): three in FP64 at orders 6 and 7 (init 66.1 and 61.2 us,
+// 70.3 and 68.9), elsewhere the compiler's own choice (0), which stops at 168 registers up to order
+// 5 and at 128 at order 2, where any stated minimum takes 160 (40.2 and 47.2 us), and does not
+// spill at order 8 (71.7 and 81.7).
+template <int K, typename T>
+constexpr int kResidualCtas = sizeof(T) == 8 && (K == 6 || K == 7) ? 3 : 0;
+
 // CTAs of one full wave of each reducing row kernel (resident CTAs per SM x SMs), per K and
 // precision ([K][0] FP64, [K][1] FP32): those kernels loop over element tiles, so one wave
 // covers any mesh and each CTA reduces once. Set by krylov_configure.
@@ -174,7 +192,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS) k_trace_in(MfOp<T> op, const
 // every reducing row kernel it runs as one wave of CTAs, each taking element tiles
 // blockIdx.x, blockIdx.x + gridDim.x, ... and reducing once.
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf_init(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs) {
+__global__ void __launch_bounds__(Rows<K>::THREADS, kResidualCtas<K, T>) k_mf_init(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs) {
     __shared__ RowScratch<K, T> sm[Rows<K>::WARPS];
     const int ntiles = (int)rgrid_of<K>(op.g.N);
     double part[2] = {0.0, 0.0};
@@ -459,12 +477,9 @@ __device__ __forceinline__ void staged_apply_loop(const MfOp<float>& op, const f
 
 // v = A ph; alpha = rho / (rhat, v); element moments of v. ST: the FP32 loop with staged
 // inputs (dynamic shared memory ApplyStage<K>::CTA_BYTES).
-// (FP32: at most 128 registers, four CTAs per SM. FP64: at most 168, three: without a limit the
-// compiler takes up to 252 and two CTAs are left to hide the loads. 256 x 512 O-grid at K = 6,
-// us per launch: 130 with two CTAs, 116 with three, 146 with four, which spill; K = 7 on 512 x 512
-// elements 325, 303, 397; K = 5 on 14,625 elements 21.9, 20.0, 22.4)
+// (registers: kOperatorCtas)
 template <int K, typename T, bool ST = false>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
+__global__ void __launch_bounds__(Rows<K>::THREADS, kOperatorCtas<K, T>)
     k_mf_v(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs) {
     KrylovScalars* sc = rs.sc;
     // the flag is uniform over the grid (only this kernel's last CTA writes it, after every
@@ -516,9 +531,8 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
 }
 
 // t = A sh; omega = (t, s) / (t, t). ST as in k_mf_v.
-// (registers as k_mf_v)
 template <int K, typename T, bool ST = false>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 4 : 3)
+__global__ void __launch_bounds__(Rows<K>::THREADS, kOperatorCtas<K, T>)
     k_mf_t(MfOp<T> op, BicgVectors<T> v, ReduceScratch rs) {
     KrylovScalars* sc = rs.sc;
     if (sc->done || sc->s_exit) return;  // uniform
@@ -643,7 +657,7 @@ __global__ void k_set_loop(const KrylovScalars* sc, cudaGraphConditionalHandle h
 
 // r = b - A x (FP64 refinement residual); ||r||^2 -> rnorm2, ||b||^2 -> bnorm2
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf_residual(MfOp<T> op, const double* __restrict__ b,
+__global__ void __launch_bounds__(Rows<K>::THREADS, kResidualCtas<K, T>) k_mf_residual(MfOp<T> op, const double* __restrict__ b,
                                                                    const T* __restrict__ x, const T* __restrict__ xtv,
                                                                    const T* __restrict__ xtg, double* __restrict__ r,
                                                                    ReduceScratch rs) {
@@ -686,8 +700,10 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3) k_mf
 // programmatic primary (mf_apply_op): everything else is loaded while that kernel still runs,
 // and the traces (read through L2, since they are being written) after it has ended. A call
 // on 9,216 elements at K = 5 is bound by the two launches and the host's synchronisation.
+// Registers: the compiler's own choice (a minimum of three CTAs an SM: K = 2 on 500^2 elements 30.2
+// us, without it 22.7; K = 6 on 256^2 48.9 and 38.8; K = 8 on 200^2 62.8 and 47.9).
 template <int K, typename T>
-__global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3)
+__global__ void __launch_bounds__(Rows<K>::THREADS)
     k_mf_apply(MfOp<T> op, const T* __restrict__ x, const T* xtv, const T* xtg, T* __restrict__ y) {
     __shared__ RowScratch<K, T> sm[Rows<K>::WARPS];
     const RowIdx<K> ix(op.g.N, blockIdx.x);
@@ -702,9 +718,10 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 1 : 3)
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");  // returns at once without a primary
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-        in.ntv[f] = ix.active ? __ldcg(xtv + q4 + f) : T(0);
-        in.ntg[f] = ix.active ? __ldcg(xtg + q4 + f) : T(0);
+    for (int f = 0; f < 4; ++f) in.ntv[f] = in.ntg[f] = T(0);
+    if (ix.active) {
+        load4_cg<T>(xtv + q4, in.ntv);
+        load4_cg<T>(xtg + q4, in.ntg);
     }
     T yy[K];
     row_apply_core<K, T>(op, in, sm[ix.warp], ix, yy);
@@ -970,6 +987,7 @@ __global__ void k_axpy_f2d(const float* e, double* x, size_t n) {
 }
 
 // ---------------------------------------------------------------- launchers
+#ifndef HO2D_KSWITCH  // (a build of a few orders only, to look at their registers, defines its own)
 #define HO2D_KSWITCH(K, CALL)                              \
     switch (K) {                                           \
         case 1: { constexpr int KK = 1; CALL; } break;      \
@@ -982,6 +1000,7 @@ __global__ void k_axpy_f2d(const float* e, double* x, size_t n) {
         case 8: { constexpr int KK = 8; CALL; } break;      \
         default: return cudaErrorInvalidValue;             \
     }
+#endif
 
 
 int krylov_max_blocks(int K, int N) {

@@ -146,6 +146,26 @@ __device__ __forceinline__ void load4(const T* __restrict__ p, T (&v)[4]) {
     }
 }
 
+// The same through L2 alone (ld.cg): values that another kernel may still have been writing when
+// this one started.
+template <typename T>
+__device__ __forceinline__ void load4_cg(const T* p, T (&v)[4]) {
+    if constexpr (sizeof(T) == 4) {
+        const float4 q = __ldcg(reinterpret_cast<const float4*>(p));
+        v[0] = q.x;
+        v[1] = q.y;
+        v[2] = q.z;
+        v[3] = q.w;
+    } else {
+        const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
+        const double2 c = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+        v[0] = a.x;
+        v[1] = a.y;
+        v[2] = c.x;
+        v[3] = c.y;
+    }
+}
+
 __device__ __forceinline__ void load4i(const int* __restrict__ p, int (&v)[4]) {
     const int4 q = __ldg(reinterpret_cast<const int4*>(p));
     v[0] = q.x;
