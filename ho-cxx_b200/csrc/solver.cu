@@ -709,21 +709,16 @@ Error Solver::poisson_solve() {
         const MfOp<double> A = make_op<double>(d, mesh_, K, false);
         const BicgVectors<double> v = krylov_vectors<double>(d, d.psi64.as<double>(), d.rhs.as<double>());
         int it = 0;
-        // Stopped a margin below the tolerance. What this preconditioner's last iterates leave of
-        // the residual sits in the few elements at a re-entrant corner, whose wall vorticity it
-        // reaches undiluted, and nearly none of it in the smooth modes. On the backward-facing
-        // step (14,625 quads, K = 5, 6 steps) the vorticity's error is 5.3e-10 (2-norm) stopped
-        // at 1e-12 and 1.6e-10 at 3e-13, for one more iteration a solve; on the 256 x 512
-        // cylinder O-grid 4.1e-11 and 8.1e-12 (4.8e-11 stopped at 1e-12 with element constants
-        // as the coarse space). Not below 1e-13, where FP64 residuals round off.
-        const double stop = std::min(tol_, std::max(0.3 * tol_, 1e-13));
-        HO2D_TRY(run(A, v, d.pc64, stop, it, d.graph64));
+        HO2D_TRY(run(A, v, d.pc64, solve_target(), it, d.graph64));
         last_iters_ += it;
         const double bn = d.h_sc->bnorm2, rn = d.h_sc->rnorm2;
         finite = std::isfinite(bn) && std::isfinite(rn);
         last_res_ = bn > 0 ? std::sqrt(rn / bn) : 0.0;
         return {0, ""};
     };
+    // what the refinement of the mixed modes aims at; one that ends above it is accepted up to the
+    // tolerance itself
+    const double target = stage32_ ? tol_ : solve_target();
     if (!krylov32_) {
         HO2D_TRY(fp64_solve());
     } else if (use_graphs_) {
@@ -746,7 +741,7 @@ Error Solver::poisson_solve() {
         }
         // the refinement's controls travel in the device scalars (the stream is idle: every
         // earlier read of h_sc was synchronised)
-        d.h_sc->tol_outer = tol_;
+        d.h_sc->tol_outer = target;
         d.h_sc->inner_tol = inner_tol_;
         d.h_sc->max_sweeps = max_sweeps_;
         static_assert(offsetof(KrylovScalars, inner_tol) == offsetof(KrylovScalars, tol_outer) + sizeof(double) &&
@@ -774,7 +769,6 @@ Error Solver::poisson_solve() {
         const MfOp<double> A64 = make_op<double>(d, mesh_, K, false);
         const MfOp<float> A32 = make_op<float>(d, mesh_, K, true);
         const BicgVectors<float> v = krylov_vectors<float>(d, d.kv[8].as<float>(), d.kv[9].as<float>());
-        bool stalled = false;
         for (;; ++sweeps) {
             HO2D_CUDA(mf_residual<double>(A64, d.rhs.as<double>(), d.psi64.as<double>(), d.kxtv.as<double>(),
                                           d.kxtg.as<double>(), d.rres.as<double>(), rs, d.stream),
@@ -791,30 +785,26 @@ Error Solver::poisson_solve() {
                 last_res_ = 0.0;
                 break;
             }
-            if (rn <= tol_ * tol_ * bn || sweeps >= max_sweeps_) break;
-            if (sweeps > 0 && !(last_res_ <= 0.5 * prev)) {  // the same stall rule as the graph
-                stalled = true;
-                break;
-            }
+            if (rn <= target * target * bn || sweeps >= max_sweeps_) break;
+            if (sweeps > 0 && !(last_res_ <= 0.5 * prev)) break;  // the same stall rule as the graph
             HO2D_CUDA(launch_copy_d2f(d.rres.as<double>(), d.kv[9].as<float>(), nv, d.stream), "d2f");
             HO2D_CUDA(cudaMemsetAsync(d.kv[8].get(), 0, nv * sizeof(float), d.stream), "memset");
             launches_ += 1;
             // ask the inner solve for no more reduction than this sweep needs: the last
             // sweep typically needs one order of magnitude, not inner_tol_'s four
-            const double need = 0.3 * tol_ / last_res_;
+            const double need = 0.3 * target / last_res_;
             const double itol = std::min(0.5, std::max(inner_tol_, need));
             int it = 0;
             HO2D_TRY(run(A32, v, d.pc32, itol, it, d.graph32));
             last_iters_ += it;
             if (!krylov_usable(*d.h_sc)) {
-                stalled = true;
                 ++sweeps;
                 break;
             }
             HO2D_CUDA(launch_axpy_f2d(d.kv[8].as<float>(), d.psi64.as<double>(), nv, d.stream), "axpy");
             launches_ += 1;
         }
-        if (finite && (stalled || !(last_res_ <= tol_))) {
+        if (finite && !(last_res_ <= tol_)) {
             ++fp64_finishes_;
             refined_res = last_res_;
             HO2D_TRY(fp64_solve());

@@ -1,6 +1,7 @@
 // solver.hpp -- one solver instance: host setup tables plus everything resident on the GPU.
 #pragma once
 
+#include <algorithm>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -216,6 +217,18 @@ class Solver {
     std::vector<double> open_normal_;         // [N_eb][K][2] unit outward normal on open edges
     std::vector<double> h_open_[6];           // host copies of the open-boundary data (start/end)
     double tol_ = 1e-12;
+    // The residual that a solve aims at: a tenth of the tolerance, not below 1e-13, where FP64
+    // residuals round off. What the vertex coarse space's last iterates leave of the residual sits
+    // in the few elements at a re-entrant corner, whose wall vorticity it reaches undiluted, and
+    // nearly none of it in the smooth modes; element constants left it evenly spread. Errors of the
+    // vorticity (2-norm and largest, against solves to 1e-14) with element constants stopped at the
+    // tolerance 1e-12, with the vertex space at 0.3 of it (FP64) or at it (refinement), and at a
+    // tenth: backward-facing step (14,625 quads, K = 5, 6 steps) FP64 7.5e-11 4.5e-9, 1.4e-10
+    // 1.7e-8, 3.6e-11 4.4e-9; HO2D_MIXED_KRYLOV 2.8e-11 1.5e-9, 9.3e-11 1.3e-8, 4.4e-12 5.5e-10;
+    // 64 x 128 cylinder O-grid, K = 5, HO2D_MIXED_KRYLOV 9.3e-14, 6.5e-13, 3.6e-14. It costs an
+    // iteration or two a solve (the step 50.7 -> 53.3 ms FP64, 36.1 -> 39.0 ms). HO2D_MIXED's
+    // refinement stops at the tolerance: its FP32 stages leave 7e-9 there.
+    double solve_target() const { return std::min(tol_, std::max(0.1 * tol_, 1e-13)); }
     int max_iter_ = 500;
     int last_iters_ = 0, prev_iters_ = 8;
     double last_res_ = 0.0;
