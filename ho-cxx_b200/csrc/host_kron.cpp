@@ -66,9 +66,9 @@ void kron_apply(const KronFit& f, const double* r, double* z) {
 
 double kron_defect(const KronFit& f, const double* D) {
     const int K2 = f.K * f.K;
-    std::vector<double> E((size_t)K2 * K2);
+    std::vector<double> E((size_t)K2 * K2), x(K2), y(K2);
     const KronFitHD h = to_hd(f);
-    return kf_defect(h, Str<double>{const_cast<double*>(D), 1}, Str<double>{E.data(), 1});
+    return kf_defect(h, Str<double>{const_cast<double*>(D), 1}, E.data(), K2, x.data(), y.data(), 0, 1, [] {});
 }
 
 void kron_store(const KronFit* f, double defect, int el, KronSmoother& ks) {

@@ -1,6 +1,6 @@
 // kron_fit.hpp -- the Kronecker-sum fit of an element's diagonal Poisson block, as one
-// source for the host (host_kron.cpp) and the device (setup_device.cu, one element per
-// thread).
+// source for the host (host_kron.cpp) and the device (setup_device.cu: the fit by one thread
+// an element, its defect by one warp).
 //
 // The diagonal block D (K^2 x K^2, row ij = (j, i), j along eta) is fitted in the least-
 // squares sense by I (x) Ax + Ay (x) I, i.e. D[(j,i),(l,k)] ~ delta_jl Ax[i][k] + Ay[j][l]
@@ -291,36 +291,45 @@ HO2D_ASM_HD inline void kf_apply(const KronFitHD& f, const double* r, double* z)
 }
 
 // ||I - M D||_2 of the fitted inverse M against D ([ij][rs] view), by 100 steps of power
-// iteration on E^T E (an estimate from below; it serves as a threshold); E is K^4 scratch.
-HO2D_ASM_HD inline double kf_defect(const KronFitHD& f, Str<double> D, Str<double> E) {
+// iteration on E^T E (an estimate from below; it serves as a threshold). Shared by `lanes`
+// workers (the host: one): worker `lane` forms columns lane, lane + lanes, ... of E and sums those
+// rows and columns of each product, every sum in the order 0 .. K^2 - 1, so the result's bits
+// do not depend on the number of workers. E: K^2 rows of `pitch` values; x, y: K^2 values; sync
+// separates the workers' phases.
+template <class Sync>
+HO2D_ASM_HD inline double kf_defect(const KronFitHD& f, Str<double> D, double* E, int pitch, double* x, double* y,
+                                    int lane, int lanes, Sync sync) {
     const int K = f.K, K2 = K * K;
     double col[kKronMaxK * kKronMaxK], z[kKronMaxK * kKronMaxK];
     // E = I - M D, column c = e_c - M (D e_c)
-    for (int c = 0; c < K2; ++c) {
+    for (int c = lane; c < K2; c += lanes) {
         for (int r = 0; r < K2; ++r) col[r] = D[(long long)r * K2 + c];
         kf_apply(f, col, z);
-        for (int r = 0; r < K2; ++r) E[(long long)r * K2 + c] = (r == c ? 1.0 : 0.0) - z[r];
+        for (int r = 0; r < K2; ++r) E[r * pitch + c] = (r == c ? 1.0 : 0.0) - z[r];
+        x[c] = 1.0;
     }
-    double x[kKronMaxK * kKronMaxK], y[kKronMaxK * kKronMaxK];
-    for (int i = 0; i < K2; ++i) x[i] = 1.0;
     double sigma2 = 0.0;
     for (int it = 0; it < 100; ++it) {
-        for (int r = 0; r < K2; ++r) {
+        sync();
+        for (int r = lane; r < K2; r += lanes) {
             double s = 0.0;
-            for (int c = 0; c < K2; ++c) s += E[(long long)r * K2 + c] * x[c];
+            for (int c = 0; c < K2; ++c) s += E[r * pitch + c] * x[c];
             y[r] = s;
         }
-        for (int c = 0; c < K2; ++c) {
+        sync();
+        for (int c = lane; c < K2; c += lanes) {
             double s = 0.0;
-            for (int r = 0; r < K2; ++r) s += E[(long long)r * K2 + c] * y[r];
+            for (int r = 0; r < K2; ++r) s += E[r * pitch + c] * y[r];
             x[c] = s;
         }
+        sync();
         double nrm = 0.0;
         for (int i = 0; i < K2; ++i) nrm += x[i] * x[i];
         nrm = sqrt(nrm);
         if (!(nrm > 0.0) || !kf_finite(nrm)) return nrm == 0.0 ? 0.0 : INFINITY;
         sigma2 = nrm;  // ||E^T E x|| with ||x|| = 1 from the second step on
-        for (int i = 0; i < K2; ++i) x[i] /= nrm;
+        sync();
+        for (int i = lane; i < K2; i += lanes) x[i] /= nrm;
     }
     return sqrt(sigma2);
 }

@@ -64,28 +64,69 @@ __global__ void __launch_bounds__(128) k_assemble(int el0, int n, AsmBases B, As
 }
 
 // ---------------------------------------------------------------- Kronecker-sum fit
-// One thread per element: the fit of its filtered diagonal block (diag [n][K4], this chunk's) and
-// its defect ||I - M D||_2 (E: K4 interleaved scratch); the factors [vx vxi vy vyi lx ly] of a
-// kept fit at el * stride in FP64 and FP32, each when asked for; zeros, exact[el] = 1 and
-// kx[el] = el where the exact block stays (kx[el] = -1 elsewhere).
+// One thread per element: the fit of its filtered diagonal block (diag [n][K4], this chunk's); the
+// factors [vx vxi vy vyi lx ly] at t * stride, exact[el] = 1 where the fit failed.
 __global__ void __launch_bounds__(128) k_kron_fit(int el0, int n, int K, const double* __restrict__ diag,
-                                                  double* __restrict__ scratch, double* __restrict__ f64,
-                                                  long long s64, float* __restrict__ f32, long long s32,
-                                                  unsigned char* __restrict__ exact, int* __restrict__ kx) {
+                                                  double* __restrict__ fac, long long stride,
+                                                  unsigned char* __restrict__ exact) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
-    const int el = el0 + t, K2 = K * K, K4 = K2 * K2, per = 4 * K2 + 2 * K;
-    const Str<double> D{const_cast<double*>(diag) + (size_t)t * K4, 1};
+    const int K2 = K * K;
     KronFitHD f;
-    const bool ok = kf_fit(K, D, f);
-    const double defect = ok ? kf_defect(f, D, Str<double>{scratch + t, n}) : 0.0;
-    const bool ex = !ok || !(defect <= kKronDefectMax);
-    exact[el] = ex ? 1 : 0;
-    if (kx) kx[el] = ex ? el : -1;
+    exact[el0 + t] = kf_fit(K, Str<double>{const_cast<double*>(diag) + (size_t)t * K2 * K2, 1}, f) ? 0 : 1;
     const double* src[4] = {f.vx, f.vxi, f.vy, f.vyi};
-    for (int i = 0; i < per; ++i) {
-        const double v = ex ? 0.0 : i < 4 * K2 ? src[i / K2][i % K2] : i < 4 * K2 + K ? f.lx[i - 4 * K2] : f.ly[i - 4 * K2 - K];
-        if (f64) f64[(size_t)el * s64 + i] = v;
+    double* o = fac + (size_t)t * stride;
+    for (int i = 0; i < 4 * K2; ++i) o[i] = src[i / K2][i % K2];
+    for (int i = 0; i < K; ++i) {
+        o[4 * K2 + i] = f.lx[i];
+        o[4 * K2 + K + i] = f.ly[i];
+    }
+}
+
+// Shared memory of k_kron_defect: E with one value of padding a row (a warp's rows then lie in
+// different banks), x and y, the factors.
+__host__ __device__ constexpr int kron_defect_bytes(int K) {
+    return (K * K * (K * K + 1) + 2 * K * K) * (int)sizeof(double) + (int)sizeof(KronFitHD);
+}
+
+// One warp per element: the fit's defect ||I - M D||_2, and with it whether the element keeps its
+// factors: as they are in fac and, with f32, in FP32 at el * s32; zeros in both, exact[el] = 1 and
+// kx[el] = el where the exact block stays (kx[el] = -1 elsewhere).
+// The defect is 200 products with a K^2 x K^2 matrix, a serial chain. One thread an element read
+// it from global memory and was bound by that latency at any number of elements: setup of 65,536
+// elements at K = 8 took 3.4 s more with the fit than without. A warp holds the matrix in shared
+// memory and sums K^2 rows side by side.
+__global__ void __launch_bounds__(32) k_kron_defect(int el0, int K, const double* __restrict__ diag,
+                                                    double* __restrict__ fac, long long stride,
+                                                    float* __restrict__ f32, long long s32,
+                                                    unsigned char* __restrict__ exact, int* __restrict__ kx) {
+    extern __shared__ double sh[];
+    const int t = blockIdx.x, el = el0 + t, lane = threadIdx.x, K2 = K * K, per = 4 * K2 + 2 * K;
+    double *E = sh, *x = E + K2 * (K2 + 1), *y = x + K2;
+    KronFitHD& f = *reinterpret_cast<KronFitHD*>(y + K2);
+    double* o = fac + (size_t)t * stride;
+    bool ex = exact[el] != 0;
+    if (!ex) {
+        double* dst[4] = {f.vx, f.vxi, f.vy, f.vyi};
+        for (int i = lane; i < 4 * K2; i += 32) dst[i / K2][i % K2] = o[i];
+        for (int i = lane; i < K; i += 32) {
+            f.lx[i] = o[4 * K2 + i];
+            f.ly[i] = o[4 * K2 + K + i];
+        }
+        if (lane == 0) f.K = K;
+        __syncwarp();
+        const double defect = kf_defect(f, Str<double>{const_cast<double*>(diag) + (size_t)t * K2 * K2, 1}, E, K2 + 1, x, y,
+                                        lane, 32, [] { __syncwarp(); });
+        ex = !(defect <= kKronDefectMax);
+    }
+    __syncwarp();
+    if (lane == 0) {
+        exact[el] = ex ? 1 : 0;
+        if (kx) kx[el] = ex ? el : -1;
+    }
+    for (int i = lane; i < per; i += 32) {
+        const double v = ex ? 0.0 : o[i];
+        if (ex) o[i] = v;
         if (f32) f32[(size_t)el * s32 + i] = (float)v;
     }
 }
@@ -333,8 +374,9 @@ Error Solver::assemble_device(bool kron32) {
     if (fit) HO2D_CUDA(ddiag.alloc((size_t)chunk * K4 * sizeof(double)), "alloc diagonal blocks");
     const int fper = 4 * K2 + 2 * K;
     const long long s64 = padded_count(fper, 8), s32 = padded_count(fper, 4);
-    DeviceBuffer dex;
+    DeviceBuffer dex, dfac;
     HO2D_CUDA(dex.alloc((size_t)N), "alloc exact flags");
+    if (fit && !kron64) HO2D_CUDA(dfac.alloc((size_t)chunk * s64 * sizeof(double)), "alloc Kronecker factors");
     if (kron64) {
         HO2D_CUDA(d.kron64.alloc(((size_t)N * s64 + 1) * sizeof(double)), "alloc Kronecker factors");
         HO2D_CUDA(cudaMemsetAsync(d.kron64.get(), 0, d.kron64.bytes(), d.stream), "memset");
@@ -351,11 +393,11 @@ Error Solver::assemble_device(bool kron32) {
                                                           dnnz.as<unsigned long long>());
         HO2D_CUDA(cudaGetLastError(), "block assembly");
         if (!fit) continue;
-        k_kron_fit<<<(n + 127) / 128, 128, 0, d.stream>>>(el0, n, K, ddiag.as<double>(), scratch.as<double>(),
-                                                          kron64 ? d.kron64.as<double>() : nullptr, s64,
-                                                          kron32 ? d.kron_f.as<float>() : nullptr, s32,
-                                                          dex.as<unsigned char>(),
-                                                          kron64 ? d.kron64_x.as<int>() : nullptr);
+        double* fac = kron64 ? d.kron64.as<double>() + (size_t)el0 * s64 : dfac.as<double>();
+        k_kron_fit<<<(n + 127) / 128, 128, 0, d.stream>>>(el0, n, K, ddiag.as<double>(), fac, s64, dex.as<unsigned char>());
+        k_kron_defect<<<n, 32, kron_defect_bytes(K), d.stream>>>(
+            el0, K, ddiag.as<double>(), fac, s64, kron32 ? d.kron_f.as<float>() : nullptr, s32, dex.as<unsigned char>(),
+            kron64 ? d.kron64_x.as<int>() : nullptr);
         HO2D_CUDA(cudaGetLastError(), "Kronecker-sum fit");
     }
     HO2D_CUDA(cudaStreamSynchronize(d.stream), "block assembly");
