@@ -305,11 +305,17 @@ cudaError_t dense_invert_device(double* a, int n, int w, cudaStream_t s, bool* s
     return cudaSuccess;
 }
 
-// Blocks that stay in L2 are read from there as fast, and the fit, a serial chain of about 10 ms
-// in each thread, would be most of a small mesh's setup: the FP64 smoother keeps the exact
-// blocks below kKronMinBytes of them (FP64 solves of 4,096 elements at K = 5, 20 MB: fine
-// smoothing 14.2 us with blocks, 12.0 with factors; 14,625 elements, 73 MB: 26.9 and 16.6).
+// Where the FP64 smoother takes Kronecker-sum factors: orders at which they are fewer values than
+// the block (4 K^2 + 2 K against K^4, so from order 3 on: at order 2 they are 20 against 16, and
+// fine smoothing of 700 x 700 elements took 40.4 us with factors, 33.5 with blocks), and meshes
+// with at least kKronMinBytes of blocks. Blocks that stay in L2 are read from there nearly as
+// fast (FP64 solves of 4,096 elements at K = 5, 20 MB: fine smoothing 14.2 us with blocks, 12.0
+// with factors; 14,625 elements, 73 MB: 26.9 and 16.6), and their solve can be one kernel.
 constexpr size_t kKronMinBytes = (size_t)48 << 20;
+static bool kron64_pays(int N, int K) {
+    const int K2 = K * K;
+    return 4 * K2 + 2 * K < K2 * K2 && (size_t)N * K2 * K2 * sizeof(double) >= kKronMinBytes;
+}
 
 // Poisson assembly on the device into the solver's buffers: inverse diagonal blocks
 // (dinv64, padded rows), block row sums (rowsum64), column sums (colsum64), the boundary
@@ -370,7 +376,7 @@ Error Solver::assemble_device(bool kron32) {
     int chunk = (int)std::min<size_t>((size_t)N, std::max<size_t>(128, ((size_t)2 << 30) / per));
     chunk = (chunk + 127) / 128 * 128;
     HO2D_CUDA(scratch.alloc((size_t)chunk * per), "alloc assembly scratch");
-    const bool kron64 = (size_t)N * K4 * sizeof(double) >= kKronMinBytes, fit = kron32 || kron64;
+    const bool kron64 = kron64_pays(N, K), fit = kron32 || kron64;
     if (fit) HO2D_CUDA(ddiag.alloc((size_t)chunk * K4 * sizeof(double)), "alloc diagonal blocks");
     const int fper = 4 * K2 + 2 * K;
     const long long s64 = padded_count(fper, 8), s32 = padded_count(fper, 4);

@@ -6,6 +6,7 @@ element the fit's defect alone took 0.6 s there, several times the rest of the s
 
 import time
 
+import numpy as np
 import pytest
 
 from ho2d import FP64, HO_2D, MIXED_KRYLOV, capi, meshgen
@@ -48,3 +49,16 @@ def test_fit_does_not_dominate_the_setup(tmp_path):
             s.close()
         times.append(best)
     assert times[1] <= 2.0 * times[0], times
+
+
+def test_order_2_keeps_blocks(tmp_path):
+    """At order 2 the factors are more values than the block (20 and 16): the FP64 smoother reads
+    blocks also on a mesh with more than 48 MB of them."""
+    n = 632
+    s = solver(meshgen.make_case("cavityj%d" % n, str(tmp_path), knod=2, steps=1), FP64)
+    s.setup()
+    s.set_vorticity(np.random.Generator(np.random.PCG64(3)).standard_normal((n * n, 2, 2)))
+    s.Euler_time_integrate(0.0)
+    data = s.profile_krylov(2)["smoother"][1] / (n * n) - 4.5 * 4 * 8  # bytes an element beside the vectors
+    s.close()
+    assert data == 16 * 8, data
