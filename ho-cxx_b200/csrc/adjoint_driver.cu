@@ -82,6 +82,51 @@ Error Solver::adjoint_prepare() {
     return {0, ""};
 }
 
+// The transposed copy of the inverse blocks `dinv` in precision gi (0 FP64, 1 FP32), made once. It is
+// as large as the blocks, the largest array of a solver by far (5.0 GB in FP64 on 512 x 512
+// elements at K = 7), so it is made only where that leaves as much memory free; elsewhere the smoother
+// reads the blocks in place (HO2D_ADJOINT_COPY=0 asks for that). A gradient on 64 x 64 elements at
+// K = 5 (4 steps) takes 80 ms with the copy and 82 without, on 96 x 96 at K = 7 (2 steps) 127 and 170.
+template <typename T>
+Error Solver::adjoint_blocks(const T* dinv, int gi) {
+    AdjointState& a = *adj_;
+    if (a.dinvT[gi].get() || a.in_place[gi]) return {0, ""};
+    DeviceState& d = *d_;
+    const int N = mesh_.n_el, K = in_.knod;
+    const size_t bytes = ((size_t)N * padded_count(K * K * K * K, (int)sizeof(T)) + 1) * sizeof(T);
+    const char* e = std::getenv("HO2D_ADJOINT_COPY");
+    size_t room = 0, total = 0;
+    HO2D_CUDA(cudaMemGetInfo(&room, &total), "cudaMemGetInfo");
+    a.in_place[gi] = (e && std::string(e) == "0") || room < 2 * bytes;
+    if (!a.in_place[gi] && a.dinvT[gi].alloc(bytes) != cudaSuccess) {
+        cudaGetLastError();
+        a.in_place[gi] = true;
+    }
+    if (a.in_place[gi]) return {0, ""};
+    HO2D_CUDA(cudaMemsetAsync(a.dinvT[gi].get(), 0, bytes, d.stream), "memset");
+    HO2D_CUDA(transpose_blocks<T>(N, K, dinv, a.dinvT[gi].as<T>(), d.stream), "transposed blocks");
+    launches_ += 1;
+    return {0, ""};
+}
+
+// An allocation of the adjoint's time loop; the transposed copies give way to it.
+Error Solver::adjoint_alloc(DeviceBuffer& b, size_t bytes, const char* what) {
+    AdjointState& a = *adj_;
+    cudaError_t e = b.alloc(bytes);
+    if (e == cudaErrorMemoryAllocation && (a.dinvT[0].get() || a.dinvT[1].get())) {
+        cudaGetLastError();
+        for (int gi = 0; gi < 2; ++gi) {
+            if (!a.dinvT[gi].get()) continue;
+            a.graph[gi].reset();
+            a.dinvT[gi].reset();
+            a.in_place[gi] = true;
+        }
+        e = b.alloc(bytes);
+    }
+    HO2D_CUDA(e, what);
+    return {0, ""};
+}
+
 // BiCGSTAB on A^T x = b in precision T to relative tolerance tol; x starts at zero. The
 // forward solver's iteration (krylov.cu) on the transposed operator: D^-T for D^-1, and the
 // coarse space's interpolation and restriction exchanged.
@@ -89,18 +134,12 @@ template <typename T>
 Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
     DeviceState& d = *d_;
     AdjointState& a = *adj_;
-    const int N = mesh_.n_el, K = in_.knod;
-    DeviceBuffer& dinvT = f32 ? a.dinvT32 : a.dinvT64;
+    const int K = in_.knod, gi = f32 ? 1 : 0;
     MfOp<T> op = make_op<T>(d, mesh_, K, f32);
-    if (!dinvT.get()) {
-        HO2D_CUDA(dinvT.alloc(((size_t)N * padded_count(K * K * K * K, (int)sizeof(T)) + 1) * sizeof(T)),
-                  "alloc transposed blocks");
-        HO2D_CUDA(cudaMemsetAsync(dinvT.get(), 0, dinvT.bytes(), d.stream), "memset");
-        HO2D_CUDA(transpose_blocks<T>(N, K, op.dinv, dinvT.as<T>(), d.stream), "transposed blocks");
-        launches_ += 1;
-    }
+    HO2D_TRY(adjoint_blocks<T>(op.dinv, gi));
     op.transposed = 1;
-    op.dinv = dinvT.as<T>();
+    op.dinv_in_place = a.in_place[gi] ? 1 : 0;
+    if (!op.dinv_in_place) op.dinv = a.dinvT[gi].as<T>();
     op.dinv_bf16 = nullptr;
     op.kron_f = op.kron_exact = nullptr;
     op.kron_x = nullptr;
@@ -128,7 +167,6 @@ Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
     if (use_graphs_) {
         // one launch of the captured solve (init and a device-side while loop); the graph
         // bakes in the operands, so it is recaptured when they change
-        const int gi = f32 ? 1 : 0;
         SolveGraph& sg = a.graph[gi];
         if (!sg.exec || sg.max_iter != max_iter_ || a.graph_x[gi] != (const void*)x || a.graph_b[gi] != (const void*)b) {
             sg.reset();
@@ -300,7 +338,7 @@ Error Solver::stage_adjoint(double coeff, const double* lam_k, double* lam_w, do
     AdjointState& a = *adj_;
     const size_t nv = (size_t)mesh_.n_el * in_.knod * in_.knod, nb = (size_t)mesh_.n_eb * in_.knod;
     if (stage32_) {  // the FP32 stage input kept, and widened in place for the FP64 stage
-        if (a.w32_save.bytes() < nv * 4) HO2D_CUDA(a.w32_save.alloc(nv * 4), "alloc");
+        if (a.w32_save.bytes() < nv * 4) HO2D_TRY(adjoint_alloc(a.w32_save, nv * 4, "alloc"));
         HO2D_CUDA(cudaMemcpyAsync(a.w32_save.get(), d.w_stage.get(), nv * 4, cudaMemcpyDeviceToDevice, d.stream),
                   "copy");
         HO2D_CUDA(launch_copy_f2d(a.w32_save.as<float>(), d.w_stage.as<double>(), nv, d.stream), "f2d");
@@ -379,7 +417,7 @@ Error Solver::adjoint_forward(int nsteps, int ckpt_every) {
     }
     while ((int)a.ckpt.size() < nck) {
         std::unique_ptr<DeviceBuffer> b(new DeviceBuffer);
-        HO2D_CUDA(b->alloc(nv * wb), "alloc checkpoint");
+        HO2D_TRY(adjoint_alloc(*b, nv * wb, "alloc checkpoint"));
         a.ckpt.push_back(std::move(b));
     }
     a.nsteps = -1;  // valid again once the sweep completes
@@ -412,8 +450,8 @@ Error Solver::adjoint_backward(const double* dJ_dw, double* grad_w0, double* gra
     const size_t wb = a.state_bytes;
     const size_t seg_bytes = (size_t)every * ns * nv * wb;
     if (a.seg_w.bytes() < seg_bytes) {
-        HO2D_CUDA(a.seg_w.alloc(seg_bytes), "alloc segment");
-        HO2D_CUDA(a.seg_psi.alloc(seg_bytes), "alloc segment");
+        HO2D_TRY(adjoint_alloc(a.seg_w, seg_bytes, "alloc segment"));
+        HO2D_TRY(adjoint_alloc(a.seg_psi, seg_bytes, "alloc segment"));
     }
     char* seg_w = static_cast<char*>(a.seg_w.get());
     char* seg_psi = static_cast<char*>(a.seg_psi.get());

@@ -138,6 +138,9 @@ struct MfOp {
     int staged = 0;
     // the operator is A^T: dinv and the vectors' hats are the transposed ones (the adjoint's solve)
     int transposed = 0;
+    // with transposed: dinv holds the blocks of A itself, whose transposes the smoother reads in
+    // place (slower; for meshes whose blocks have no room for a transposed copy)
+    int dinv_in_place = 0;
     // host side: a second stream and two events; when set, each coarse cycle runs on the
     // second stream beside the fine part of the smoothing step (k_post_a)
     cudaStream_t side = nullptr;

@@ -1044,6 +1044,12 @@ static void iteration_impl(const MfOp<T>& op, const BicgVectors<T>& v, const Red
     const unsigned gp = rgrid_of<K>(N);
     constexpr int tp = Rows<K>::THREADS;
     auto post_a = [&](int mode) {
+        if constexpr (TR) {
+            if (op.dinv_in_place) {
+                k_post_a<K, T, 3><<<gp, tp, PostRows<K, T, 3>::SMEM, s>>>(op, v, mg, rs, mode);
+                return;
+            }
+        }
         if constexpr (!TR) {
             if (op.kron_f) {
                 k_post_a<K, T, 2><<<gp, tp, PostRows<K, T, 2>::SMEM, s>>>(op, v, mg, rs, mode);
@@ -1155,6 +1161,8 @@ static cudaError_t configure_post() {
     };
     one(k_post_a<K, double, 0>, PostRows<K, double, 0>::SMEM);
     one(k_post_a<K, double, 2>, PostRows<K, double, 2>::SMEM);
+    one(k_post_a<K, double, 3>, PostRows<K, double, 3>::SMEM);
+    one(k_post_a<K, float, 3>, PostRows<K, float, 3>::SMEM);
     one(k_post_a<K, float, 0>, PostRows<K, float, 0>::SMEM);
     one(k_post_a<K, float, 1>, PostRows<K, float, 1>::SMEM);
     one(k_post_a<K, float, 2>, PostRows<K, float, 2>::SMEM);
@@ -1207,6 +1215,10 @@ HO2D_FUSED_DECL(fused_tr32, float);
 template <typename T>
 cudaError_t krylov_fused(const MfOp<T>& op, const BicgVectors<T>& v, const FusedScratch& fs, int max_iter,
                          const Precond<T>& pc, KrylovScalars* sc, cudaStream_t s, bool* fits) {
+    if (op.dinv_in_place) {
+        *fits = false;
+        return cudaSuccess;
+    }
     if constexpr (std::is_same<T, float>::value) {
         if (op.transposed) return fused_tr32(op, v, fs, max_iter, pc, sc, s, fits);
         if (op.kron_f) return fused_f32_kron(op, v, fs, max_iter, pc, sc, s, fits);

@@ -1,5 +1,6 @@
 // smoother.cuh -- the fine smoother's element inverse on the row-parallel mapping (rows.cuh):
-// exact blocks, BF16 blocks or Kronecker-sum factors, applied to one element vector.
+// exact blocks (or their transposes), BF16 blocks or Kronecker-sum factors, applied to one
+// element vector.
 #pragma once
 
 #include <type_traits>
@@ -10,8 +11,9 @@ namespace ho2d {
 
 // The smoother's element data (BS): 0 = inverse blocks in T; 1 = inverse blocks as BF16 bit
 // patterns (FP32 smoother); 2 = Kronecker-sum factors, with the exact blocks only for the
-// elements the fit does not approximate well (FP32 smoother). Each element's data starts on
-// a 16-byte boundary (padded_count). A warp's EPW blocks (or factor sets) are one
+// elements the fit does not approximate well; 3 = the blocks of 0 applied transposed, read where
+// they lie (the adjoint's solve without a transposed copy). Each element's data starts on a
+// 16-byte boundary (padded_count). A warp's EPW blocks (or factor sets) are one
 // contiguous span, copied into shared memory by one bulk copy when the span is at most
 // 26 KB (so a CTA's four spans leave room for two CTAs per SM); larger blocks are read
 // from global memory directly.
@@ -100,6 +102,23 @@ __device__ __forceinline__ void block_rows(const DT* blk, const T* sr, int t, T 
     }
 }
 
+// The same with the block's transpose: acc[i] = sum_r blk[t K + i][r] sr[r], r in the same order, so
+// the result has the bits that block_rows gives on a transposed copy. Each thread streams K rows of
+// the block, its neighbours the next K, so a warp's loads fall into many lines at once (the cost
+// stands at Solver::adjoint_blocks).
+template <int K, typename T>
+__device__ __forceinline__ void block_rows_transposed(const T* blk, const T* sr, int t, T (&acc)[K]) {
+    constexpr int K2 = K * K;
+#pragma unroll
+    for (int i = 0; i < K; ++i) acc[i] = T(0);
+#pragma unroll 4
+    for (int r = 0; r < K2; ++r) {
+        const T s = sr[r];
+#pragma unroll
+        for (int i = 0; i < K; ++i) acc[i] += blk[(t * K + i) * K2 + r] * s;
+    }
+}
+
 // The smoother's element inverse M (exact block, BF16 block or Kronecker-sum factors)
 // applied to one element vector held in shared memory (srow, K^2 values, [j][i]): row t of
 // M srow into acc. For BS 2 the transposes are warp-collective, so every lane runs them;
@@ -163,6 +182,8 @@ __device__ __forceinline__ void smoother_rows(const MfOp<T>& op, const typename 
             }
         }
         __syncwarp();  // zb may be reused by the caller
+    } else if constexpr (BS == 3) {
+        if (act) block_rows_transposed<K, T>(blk, srow, t, acc);
     } else {
         if (act) block_rows<K, T, typename PS::DT>(blk, srow, t, acc);
     }

@@ -175,6 +175,9 @@ class Solver {
                            DeviceBuffer& dense64, DeviceBuffer& dense32, Precond<double>& pc64, Precond<float>& pc32,
                            std::vector<int>* sizes);
     Error adjoint_prepare();
+    template <typename T>
+    Error adjoint_blocks(const T* dinv, int gi);
+    Error adjoint_alloc(DeviceBuffer& b, size_t bytes, const char* what);
     Error stage_adjoint_dev(double coeff, double* out);
     Error transposed_solve(const double* rhs, double* mu);
     Error store_state(void* dst, const double* src);

@@ -150,9 +150,11 @@ struct DeviceState {
 // Device state of the discrete adjoint, allocated on first use.
 struct AdjointState {
     bool ready = false;
-    // the transposed inverse blocks (one copy per precision, made when first used); the rest
-    // of the transposed solve's preconditioner is the forward one's
-    DeviceBuffer dinvT64, dinvT32;
+    // the transposed inverse blocks (a copy per precision, made when first used, if there is
+    // room: Solver::adjoint_blocks); the rest of the transposed solve's preconditioner is the
+    // forward one's
+    DeviceBuffer dinvT[2];
+    bool in_place[2] = {false, false};  // no copy: the blocks are read where they are
     // BiCGSTAB on A^T: r rhat p v s t ph sh (sized for FP64), slots [N][K][4]
     DeviceBuffer kv[8];
     DeviceBuffer sv, sg;
