@@ -96,10 +96,4 @@ struct KrylovScalars {
 // down in FP32, and its x may then hold anything.
 __host__ __device__ inline bool krylov_usable(const KrylovScalars& sc) { return sc.rnorm2 <= sc.bnorm2; }
 
-// A preconditioner application is skipped once the solve is done, and the second one of
-// an iteration (mode 1) also when the iteration exits early after its s update.
-__device__ __forceinline__ bool pc_skip(const KrylovScalars* sc, int mode) {
-    return sc->done || (mode == 1 && sc->s_exit);
-}
-
 }  // namespace ho2d

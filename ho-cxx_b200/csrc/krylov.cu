@@ -1205,7 +1205,6 @@ cudaError_t krylov_iteration_timed(const MfOp<T>& op, const BicgVectors<T>& v, c
     cudaError_t NAME(const MfOp<T>&, const BicgVectors<T>&, const FusedScratch&, int, const Precond<T>&,        \
                      KrylovScalars*, cudaStream_t, bool*)
 HO2D_FUSED_DECL(fused_f64, double);
-HO2D_FUSED_DECL(fused_f64_kron, double);
 HO2D_FUSED_DECL(fused_tr64, double);
 HO2D_FUSED_DECL(fused_f32_exact, float);
 HO2D_FUSED_DECL(fused_f32_bf16, float);
@@ -1226,7 +1225,12 @@ cudaError_t krylov_fused(const MfOp<T>& op, const BicgVectors<T>& v, const Fused
         return fused_f32_exact(op, v, fs, max_iter, pc, sc, s, fits);
     } else {
         if (op.transposed) return fused_tr64(op, v, fs, max_iter, pc, sc, s, fits);
-        if (op.kron_f) return fused_f64_kron(op, v, fs, max_iter, pc, sc, s, fits);
+        // factors come with at least 48 MB of blocks (kKronMinBytes, setup_device.cu), more tiles than
+        // the one-kernel solve takes at any order
+        if (op.kron_f) {
+            *fits = false;
+            return cudaSuccess;
+        }
         return fused_f64(op, v, fs, max_iter, pc, sc, s, fits);
     }
 }
