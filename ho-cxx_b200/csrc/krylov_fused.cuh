@@ -213,8 +213,8 @@ constexpr int resident_bytes() {
 }
 
 // The solve. BS: the smoother's element data (smoother.cuh); TR: the transposed operator (v.b
-// is the right-hand side and x starts at zero); One tile per CTA,
-// its element data resident in shared memory.
+// is the right-hand side and x starts at zero). CTA b works on element tile b alone, whose
+// smoother data stay in its shared memory (fused_launch: at least as many CTAs as tiles).
 template <int K, typename T, int BS, bool TR>
 __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
     k_fused_solve(const __grid_constant__ MfOp<T> op, const __grid_constant__ BicgVectors<T> v,
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
     __shared__ double red[2][NT / 32];
     __shared__ bool s_ok;
     KrylovScalars* sc = rs.sc;
-    const int N = op.g.N, ntiles = (N + R::EPC - 1) / R::EPC;
+    const int N = op.g.N, ntiles = (N + R::EPC - 1) / R::EPC, tile = blockIdx.x;  // at most one tile a CTA
     const int d = pc.nlev - 1;  // -1: no coarse level
     const double tol = __ldcg(&sc->tol);
     const unsigned char* el_data = BS == 2 ? reinterpret_cast<const unsigned char*>(op.kron_f)
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
 
     // traces of x, the initial residual's operand
     if constexpr (!TR) {
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        if (tile < ntiles) {
             const RowIdx<K> ix(N, tile);
             T row[K];
             int dst[4];
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
     // mode 2: the initial residual; 0: v = A ph; 1: t = A sh
     for (int mode = 2;;) {
         double part[2] = {0.0, 0.0};
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        if (tile < ntiles) {
             const RowIdx<K> ix(N, tile);
             const size_t p = (size_t)ix.el * K2 + ix.t * K;
             T y[K], q[K];
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
     update:
         if (mode == 3) {  // x, r and the end of the iteration
             double up[2] = {0.0, 0.0};
-            for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            if (tile < ntiles) {
                 const RowIdx<K> ix(N, tile);
                 const size_t p = (size_t)ix.el * K2 + ix.t * K;
                 T r[K];
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
         }
         auto moment = [&](int e) { return ldm(f0.a + e) + f0.cb * ldm(f0.b + e) + f0.cc * ldm(f0.c + e); };
         double sp[2] = {0.0, 0.0};
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        if (tile < ntiles) {
             const RowIdx<K> ix(N, tile);
             const int t = ix.t, el = ix.el;
             const size_t p = (size_t)el * K2 + t * K;
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
             smoother_rows<K, T, BS>(op, reinterpret_cast<const DT*>(data), reinterpret_cast<const T*>(data), kx,
                                     &sm[ix.warp].tr[0][ix.lw][0][0], sm[ix.warp].tr[1][ix.lw], t, ix.active, acc);
             if (ix.active) store_row<K, T>(v.zf + p, acc);
-            __syncwarp();  // the scratch is rewritten by the next tile
+            __syncwarp();  // the scratch is rewritten by the next phase
         }
         if (d >= 0) {
             T* f = pc.lev[0].f;
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, sizeof(T) == 4 ? 3 : 1)
             if (!sync()) return;
         }
         // z = P u0 + w zf, its traces (or its own part of A^T z)
-        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        if (tile < ntiles) {
             const RowIdx<K> ix(N, tile);
             const int t = ix.t;
             const size_t p = (size_t)ix.el * K2 + t * K;
