@@ -695,6 +695,8 @@ HO2D_HD void gather_body(const C& c, bool active, int el, const DevBases<T>& b, 
 
 // First half of y = A^T x (A the Poisson operator, psi boundary switches, homogeneous
 // values): this element's own part in dir and its neighbours' parts in their slots.
+// Host builds only: the device applies A^T by rows_transpose.cuh. It checks lap_adjoint, which the
+// stage adjoint's kernels share, against the assembled matrix.
 template <int K, typename T, class C>
 HO2D_HD void poisson_transpose_body(const C& c, bool active, int el, const FrGeom<T>& g, const DevBases<T>& b,
                                     const T* x, T* dir, T* slot_v, T* slot_g, LapAdjScratch<K, T>& s) {
