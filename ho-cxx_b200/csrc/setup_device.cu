@@ -14,6 +14,8 @@
 // in place in the row-padded FP64 storage the coarse cycle reads.
 #include <cuda_runtime.h>
 
+#include <cstdlib>
+
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -314,7 +316,9 @@ cudaError_t dense_invert_device(double* a, int n, int w, cudaStream_t s, bool* s
 constexpr size_t kKronMinBytes = (size_t)48 << 20;
 static bool kron64_pays(int N, int K) {
     const int K2 = K * K;
-    return 4 * K2 + 2 * K < K2 * K2 && (size_t)N * K2 * K2 * sizeof(double) >= kKronMinBytes;
+    const char* e = std::getenv("HO2D_KRON64_MIN");  // (a test hook: the line in bytes, for small meshes)
+    const size_t line = e ? (size_t)std::atoll(e) : kKronMinBytes;
+    return 4 * K2 + 2 * K < K2 * K2 && (size_t)N * K2 * K2 * sizeof(double) >= line;
 }
 
 // Poisson assembly on the device into the solver's buffers: inverse diagonal blocks
