@@ -161,7 +161,7 @@ Error Solver::kt_run(T* x, const T* b, bool f32, double tol, int& iters) {
     auto poll = [&]() -> Error {
         HO2D_CUDA(cudaMemcpyAsync(d.h_sc, rs.sc, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, d.stream), "poll");
         HO2D_CUDA(cudaStreamSynchronize(d.stream), "poll");
-        if (d.h_sc->dev_error) return {5, "a device-side wait for a bulk copy ran out (the GPU did not complete it)"};
+        if (d.h_sc->dev_error) return {5, kWaitRanOut};
         return {0, ""};
     };
     if (use_graphs_) {

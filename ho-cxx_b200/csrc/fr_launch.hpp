@@ -128,8 +128,9 @@ struct MfOp {
     const T* dinv;          // [N][K2][K2] inverse diagonal blocks, transposed ([rs][ij])
     // optional BF16 copy of dinv (bit patterns), read by the FP32 smoother when present
     const unsigned short* dinv_bf16 = nullptr;
-    // optional Kronecker-sum smoother (FP32): factors [N][4K^2 + 2K], the compact index of
-    // each element's exact block or -1 [N], and those exact blocks [n][K2][K2] ([rs][ij])
+    // optional Kronecker-sum smoother: factors [N][4K^2 + 2K], the index of each element's exact
+    // block or -1 [N], and the blocks it indexes [n][K2][K2] ([rs][ij]; FP32: a compact copy, FP64:
+    // dinv)
     const T* kron_f = nullptr;
     const int* kron_x = nullptr;
     const T* kron_exact = nullptr;

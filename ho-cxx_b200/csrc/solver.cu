@@ -655,7 +655,7 @@ Error Solver::poisson_solve() {
         HO2D_CUDA(cudaMemcpyAsync(d.h_sc, d.scalars.get(), sizeof(KrylovScalars), cudaMemcpyDeviceToHost, d.stream),
                   "poll");
         HO2D_CUDA(cudaStreamSynchronize(d.stream), "poll");
-        if (d.h_sc->dev_error) return {5, "a device-side wait for a bulk copy ran out (the GPU did not complete it)"};
+        if (d.h_sc->dev_error) return {5, kWaitRanOut};
         return {0, ""};
     };
     // runs BiCGSTAB to completion on (A, v); returns iterations
@@ -1223,12 +1223,14 @@ Error Solver::profile_krylov(int reps, double* ms, double* bytes) {
         if (!krylov32_ && d.kron64.get()) blk = (4.0 * K2 + 2 * K) * 8 + (double)kron64_exact_ / N * K4 * 8;
         if (krylov32_ && smoother_kind_ == 1) blk = K4 * 2;
         if (krylov32_ && smoother_kind_ == 2) blk = (4.0 * K2 + 2 * K) * 4 + (double)smoother_exact_ / N * K4 * 4;
-        bytes[0] = (double)N * (blk + 4.5 * K2 * bw);
+        // and the element moments (4 an element): p's formed from r's, v's and the last p's in mode 0
+        const double mom = coarse_bytes > 0 ? 4.0 * bw : 0.0;
+        bytes[0] = (double)N * (blk + 4.5 * K2 * bw + 0.5 * (3 + 1) * mom);
         // per element: operand, 3 metric coefficients, rhat or s, result; 4 face coefficients
-        // and 2 incoming traces per face point; 4 face codes; the element sum
-        bytes[1] = (double)N * ((6.0 * K2 + 24.0 * K) * bw + 16.0 + bw);
-        // x, ph, sh, s, t, rhat read; x and r written; the element sum of r
-        bytes[2] = (double)N * (8.0 * K2 * bw + bw);
+        // and 2 incoming traces per face point; 4 face codes; v's element moments (half the launches)
+        bytes[1] = (double)N * ((6.0 * K2 + 24.0 * K) * bw + 16.0 + 0.5 * 4.0 * bw);
+        // x, ph, sh, s, t, rhat read; x and r written; r's element moments
+        bytes[2] = (double)N * (8.0 * K2 * bw + 4.0 * bw);
         bytes[3] = coarse_bytes;
         // combination, per element: M f and the 4 coarse values read, z and its 4K face traces
         // (value, derivative) written, 4K destinations and 4 corners read

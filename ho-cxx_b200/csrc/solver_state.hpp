@@ -306,6 +306,9 @@ MfOp<T> make_op(DeviceState& d, const Mesh& m, int K, bool f32) {
     return op;
 }
 
+// what KrylovScalars::dev_error means
+constexpr char kWaitRanOut[] = "a device-side wait ran out (a bulk copy or a grid barrier that the GPU did not complete)";
+
 inline ReduceScratch reduce_scratch(DeviceState& d) {
     return {d.partials.as<double>(), d.counter.as<unsigned>(), d.scalars.as<KrylovScalars>(),
             d.fused_partials.as<double>(), d.fused_bar.as<unsigned>()};

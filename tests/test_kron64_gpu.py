@@ -24,7 +24,7 @@ def solve(inp, w0):
     s.Euler_time_integrate(0.0)
     psi, iters = s.get_streamfunction(), s.poisson_stats()[0]
     k2 = s.Knod ** 2
-    data = s.profile_krylov(1)["smoother"][1] / s.N_el - 4.5 * k2 * 8  # bytes an element beside the vectors
+    data = s.profile_krylov(1)["smoother"][1] / s.N_el - (4.5 * k2 + 8) * 8  # an element, beside vectors and moments
     s.close()
     return psi, iters, data
 

@@ -59,6 +59,6 @@ def test_order_2_keeps_blocks(tmp_path):
     s.setup()
     s.set_vorticity(np.random.Generator(np.random.PCG64(3)).standard_normal((n * n, 2, 2)))
     s.Euler_time_integrate(0.0)
-    data = s.profile_krylov(2)["smoother"][1] / (n * n) - 4.5 * 4 * 8  # bytes an element beside the vectors
+    data = s.profile_krylov(2)["smoother"][1] / (n * n) - (4.5 * 4 + 8) * 8  # an element, beside vectors and moments
     s.close()
     assert data == 16 * 8, data
