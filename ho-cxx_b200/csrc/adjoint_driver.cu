@@ -211,12 +211,12 @@ Error Solver::transposed_solve(const double* rhs, double* mu) {
     const size_t nv = (size_t)N * K * K;
     const ReduceScratch rs = reduce_scratch(d);
     bool finite = true;
-    const double target = solve_target();
+    const RefineGoal goal = refine_goal(true);
     last_adj_iters_ = 0;
     int sweeps = 0;
     if (!krylov32_) {
         int it = 0;
-        HO2D_TRY(kt_run<double>(mu, rhs, false, target, it));
+        HO2D_TRY(kt_run<double>(mu, rhs, false, solve_target(), it));
         last_adj_iters_ = it;
         const double bn = d.h_sc->bnorm2, rn = d.h_sc->rnorm2;
         finite = std::isfinite(bn) && std::isfinite(rn);
@@ -239,14 +239,14 @@ Error Solver::transposed_solve(const double* rhs, double* mu) {
             finite = std::isfinite(bn) && std::isfinite(rn);
             last_adj_res_ = bn > 0 ? std::sqrt(rn / bn) : 0.0;
             if (!finite || bn == 0.0) break;
-            if (rn <= target * target * bn || sweeps >= 30) break;
+            if (rn <= goal.accept * goal.accept * bn || sweeps >= 30) break;
             // a sweep that did not halve the residual (the forward refinement's rule) or an FP32
             // solve that broke down: the FP64 solve of the remaining residual finishes
             if (lost || (sweeps > 0 && !(last_adj_res_ <= 0.5 * prev))) {
                 if (last_adj_res_ <= tol_) break;  // above what it aimed at, but within the tolerance
                 int it = 0;
                 HO2D_TRY(kt_run<double>(a.x32.as<double>(), a.res64.as<double>(), false,
-                                        std::min(0.5, target / last_adj_res_), it));
+                                        std::min(0.5, solve_target() / last_adj_res_), it));
                 last_adj_iters_ += it;
                 last_adj_res_ *= std::sqrt(d.h_sc->rnorm2 / d.h_sc->bnorm2);
                 finite = std::isfinite(last_adj_res_);
@@ -256,7 +256,7 @@ Error Solver::transposed_solve(const double* rhs, double* mu) {
             }
             prev = last_adj_res_;
             HO2D_CUDA(launch_copy_d2f(a.res64.as<double>(), a.b32.as<float>(), nv, d.stream), "d2f");
-            const double need = 0.3 * target / last_adj_res_;
+            const double need = goal.aim / last_adj_res_;
             const double itol = std::min(0.5, std::max(inner_tol_, need));
             int it = 0;
             HO2D_TRY(kt_run<float>(a.x32.as<float>(), a.b32.as<float>(), true, itol, it));

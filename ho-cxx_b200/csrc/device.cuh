@@ -79,11 +79,11 @@ struct KrylovScalars {
     int it, done, breakdown, s_exit, zero_rhs, pad;
     double tol;  // relative tolerance of the next solve, written by the host before it starts
     // FP64 iterative refinement around the FP32 solve when it runs on the device (one graph
-    // per solve): the target on the FP64 residual, the smallest inner reduction asked of a
-    // sweep and the sweep cap (written by the host), then the sweeps done, the inner
+    // per solve): the FP64 residual that is accepted and the one that a sweep aims at, the smallest
+    // inner reduction asked of a sweep and the sweep cap (written by the host), then the sweeps done, the inner
     // iterations summed over them, the last relative FP64 residual, whether it was finite
     // and whether the right-hand side was zero (written by the device)
-    double tol_outer, inner_tol;
+    double tol_outer, aim_outer, inner_tol;
     int max_sweeps, sweeps, iters_total, finite, zero_psi;
     int dev_error;  // nonzero: a kernel's bounded wait ran out (the host reports it)
     double res;

@@ -914,8 +914,8 @@ __global__ void k_transpose_blocks(int N, int K2, int stride, const T* __restric
 // FP64 residual }. k_refine_ctl decides after every FP64 residual, with the rule the
 // host loop uses: stop on a non-finite or zero residual norm, at the target, at the sweep
 // cap, or when the last sweep did not halve the residual (stalled: the host finishes the
-// solve in FP64); otherwise ask the inner solve for max(inner_tol, 0.3 target / current)
-// relative reduction (at most 0.5), so the last sweep does not overshoot.
+// solve in FP64); otherwise ask the inner solve for max(inner_tol, aim / current) relative
+// reduction (at most 0.5), so the last sweep does not overshoot.
 __global__ void k_refine_begin(KrylovScalars* sc) {
     sc->sweeps = 0;
     sc->iters_total = 0;
@@ -944,7 +944,7 @@ __global__ void k_refine_ctl(KrylovScalars* sc, cudaGraphConditionalHandle h) {
     sc->res = res;
     sc->finite = fin;
     if (!stop) {
-        const double need = 0.3 * sc->tol_outer / res;
+        const double need = sc->aim_outer / res;
         sc->tol = fmin(0.5, fmax(sc->inner_tol, need));
         sc->sweeps += 1;
     }

@@ -716,9 +716,8 @@ Error Solver::poisson_solve() {
         last_res_ = bn > 0 ? std::sqrt(rn / bn) : 0.0;
         return {0, ""};
     };
-    // what the refinement of the mixed modes aims at; one that ends above it is accepted up to the
-    // tolerance itself
-    const double target = stage32_ ? tol_ : solve_target();
+    // (a refinement that stalls above its goal is accepted up to the tolerance itself)
+    const RefineGoal goal = refine_goal(!stage32_);
     if (!krylov32_) {
         HO2D_TRY(fp64_solve());
     } else if (use_graphs_) {
@@ -741,14 +740,15 @@ Error Solver::poisson_solve() {
         }
         // the refinement's controls travel in the device scalars (the stream is idle: every
         // earlier read of h_sc was synchronised)
-        d.h_sc->tol_outer = target;
+        d.h_sc->tol_outer = goal.accept;
+        d.h_sc->aim_outer = goal.aim;
         d.h_sc->inner_tol = inner_tol_;
         d.h_sc->max_sweeps = max_sweeps_;
-        static_assert(offsetof(KrylovScalars, inner_tol) == offsetof(KrylovScalars, tol_outer) + sizeof(double) &&
+        static_assert(offsetof(KrylovScalars, inner_tol) == offsetof(KrylovScalars, tol_outer) + 2 * sizeof(double) &&
                           offsetof(KrylovScalars, max_sweeps) == offsetof(KrylovScalars, inner_tol) + sizeof(double),
                       "refinement controls are contiguous");
         HO2D_CUDA(cudaMemcpyAsync(&d.scalars.as<KrylovScalars>()->tol_outer, &d.h_sc->tol_outer,
-                                  2 * sizeof(double) + sizeof(int), cudaMemcpyHostToDevice, d.stream),
+                                  3 * sizeof(double) + sizeof(int), cudaMemcpyHostToDevice, d.stream),
                   "refinement controls");
         HO2D_CUDA(cudaGraphLaunch(sg.exec, d.stream), "graph launch");
         HO2D_TRY(poll());
@@ -785,14 +785,14 @@ Error Solver::poisson_solve() {
                 last_res_ = 0.0;
                 break;
             }
-            if (rn <= target * target * bn || sweeps >= max_sweeps_) break;
+            if (rn <= goal.accept * goal.accept * bn || sweeps >= max_sweeps_) break;
             if (sweeps > 0 && !(last_res_ <= 0.5 * prev)) break;  // the same stall rule as the graph
             HO2D_CUDA(launch_copy_d2f(d.rres.as<double>(), d.kv[9].as<float>(), nv, d.stream), "d2f");
             HO2D_CUDA(cudaMemsetAsync(d.kv[8].get(), 0, nv * sizeof(float), d.stream), "memset");
             launches_ += 1;
             // ask the inner solve for no more reduction than this sweep needs: the last
             // sweep typically needs one order of magnitude, not inner_tol_'s four
-            const double need = 0.3 * target / last_res_;
+            const double need = goal.aim / last_res_;
             const double itol = std::min(0.5, std::max(inner_tol_, need));
             int it = 0;
             HO2D_TRY(run(A32, v, d.pc32, itol, it, d.graph32));

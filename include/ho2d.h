@@ -171,9 +171,9 @@ enum ho2d_setup_array {
 };
 int ho2d_get_poisson_setup(ho2d_solver* handle, int32_t which, int64_t len, double* buf);
 /* Poisson solve controls: relative tolerance on ||b - A psi|| / ||b|| (default 1e-12)
- * and iteration cap (default 500). HO2D_FP64, HO2D_MIXED_KRYLOV and the adjoint's transposed
- * solves aim at a tenth of it (not below 1e-13), so that the vorticity at re-entrant corners
- * is as accurate as the tolerance says; HO2D_MIXED stops at the tolerance. */
+ * and iteration cap (default 500). Solves go below it (not below 1e-13), for the vorticity at
+ * re-entrant corners: HO2D_FP64 and the adjoint in FP64 stop at a tenth of it, the refinement
+ * of HO2D_MIXED_KRYLOV and of the adjoint in the mixed modes at 0.3. HO2D_MIXED stops at it. */
 int ho2d_set_poisson_tolerance(ho2d_solver* handle, double rel_tol, int32_t max_iter);
 /* Statistics of the last Poisson solve: Krylov iterations (inner iterations summed over
  * refinement sweeps) and final relative residual. */

@@ -1,7 +1,7 @@
-"""The residual that Poisson solves end with, on the GPU. The FP64 solve, the refinement of
-HO2D_MIXED_KRYLOV and the adjoint's transposed solves aim at a tenth of the tolerance (the
-reason stands at Solver::solve_target); at 1e-9 nothing stalls, so every solve has to get there.
-HO2D_MIXED stops at the tolerance.
+"""The residual that Poisson solves end with, on the GPU: in FP64 a tenth of the tolerance, the
+adjoint's transposed solves included, in the refinement of HO2D_MIXED_KRYLOV and of the transposed
+solves 0.3 of it (the reason stands at Solver::solve_target). HO2D_MIXED stops at the tolerance.
+At 1e-9 nothing stalls, so every solve has to get there.
 """
 
 import numpy as np
@@ -16,8 +16,8 @@ TOL = 1e-9
 
 @pytest.mark.parametrize("graphs", ["1", "0"])
 @pytest.mark.parametrize("mesh,knod", [("cyl6x13", 4), ("cavityj72", 5)])  # one kernel a solve; launches
-@pytest.mark.parametrize("precision,bound", [(FP64, 0.1), (MIXED_KRYLOV, 0.1), (MIXED, 1.0)])
-def test_solves_end_below_their_target(tmp_path, monkeypatch, precision, bound, mesh, knod, graphs):
+@pytest.mark.parametrize("precision,bound,bound_transposed", [(FP64, 0.1, 0.1), (MIXED_KRYLOV, 0.3, 0.3), (MIXED, 1.0, 0.3)])
+def test_solves_end_below_their_target(tmp_path, monkeypatch, precision, bound, bound_transposed, mesh, knod, graphs):
     monkeypatch.setenv("HO2D_GRAPHS", graphs)
     s = HO_2D()
     s.read_input_file(meshgen.make_case(mesh, str(tmp_path), knod=knod, steps=1))
@@ -35,4 +35,4 @@ def test_solves_end_below_their_target(tmp_path, monkeypatch, precision, bound, 
         transposed.append(s.adjoint_stats()[1])
     s.close()
     assert max(forward) <= bound * TOL, forward
-    assert max(transposed) <= 0.1 * TOL, transposed
+    assert max(transposed) <= bound_transposed * TOL, transposed
