@@ -216,7 +216,7 @@ Error Solver::transposed_solve(const double* rhs, double* mu) {
     int sweeps = 0;
     if (!krylov32_) {
         int it = 0;
-        HO2D_TRY(kt_run<double>(mu, rhs, false, solve_target(), it));
+        HO2D_TRY(kt_run<double>(mu, rhs, false, transposed_target(), it));
         last_adj_iters_ = it;
         const double bn = d.h_sc->bnorm2, rn = d.h_sc->rnorm2;
         finite = std::isfinite(bn) && std::isfinite(rn);
@@ -246,7 +246,7 @@ Error Solver::transposed_solve(const double* rhs, double* mu) {
                 if (last_adj_res_ <= tol_) break;  // above what it aimed at, but within the tolerance
                 int it = 0;
                 HO2D_TRY(kt_run<double>(a.x32.as<double>(), a.res64.as<double>(), false,
-                                        std::min(0.5, solve_target() / last_adj_res_), it));
+                                        std::min(0.5, transposed_target() / last_adj_res_), it));
                 last_adj_iters_ += it;
                 last_adj_res_ *= std::sqrt(d.h_sc->rnorm2 / d.h_sc->bnorm2);
                 finite = std::isfinite(last_adj_res_);

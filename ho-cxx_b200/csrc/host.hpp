@@ -182,6 +182,12 @@ struct AsmCoefficients {
 AsmCoefficients assembly_coefficients(const Bases& B);
 AsmBases asm_bases(const Bases& B);
 int tensor2fem(int i, int j, int lnod_in);
+// The largest interior angle of the domain at a boundary vertex (the sum of the angles that the
+// elements have there, between their corners): pi on a straight wall, 3/2 pi at a backward-facing step.
+double largest_boundary_angle(const Mesh& m);
+// Above it a vertex counts as a re-entrant corner: 234 degrees, more than a round body meshed with seven
+// or more edges has.
+constexpr double kCornerAngle = 1.3 * 3.14159265358979323846;
 
 // Fields written by the VTK output: volume arrays [N][K][K] (vorticity, streamfunction,
 // Cartesian velocity components, the two RHS terms), boundary arrays [N_eb][K]

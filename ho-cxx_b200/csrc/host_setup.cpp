@@ -574,4 +574,24 @@ AsmCoefficients assembly_coefficients(const Bases& B) {
     return c;
 }
 
+double largest_boundary_angle(const Mesh& m) {
+    const int lin = m.lnod - 1;
+    const int corner[4] = {tensor2fem(0, 0, lin), tensor2fem(lin, 0, lin), tensor2fem(lin, lin, lin),
+                           tensor2fem(0, lin, lin)};
+    std::vector<double> angle(m.node_xy.size() / 2, -1.0);
+    for (int e = 0; e < m.n_eb; ++e)
+        for (int q = 0; q < 2; ++q) angle[m.elem_nodes[m.be_el[e]][corner[(m.be_side[e] + q) % 4]]] = 0.0;
+    for (int el = 0; el < m.n_el; ++el)
+        for (int c = 0; c < 4; ++c) {
+            const int v = m.elem_nodes[el][corner[c]];
+            if (angle[v] < 0.0) continue;
+            const double* p = &m.node_xy[(size_t)v * 2];
+            const double* a = &m.node_xy[(size_t)m.elem_nodes[el][corner[(c + 1) % 4]] * 2];
+            const double* b = &m.node_xy[(size_t)m.elem_nodes[el][corner[(c + 3) % 4]] * 2];
+            const double ax = a[0] - p[0], ay = a[1] - p[1], bx = b[0] - p[0], by = b[1] - p[1];
+            angle[v] += std::atan2(ax * by - ay * bx, ax * bx + ay * by);
+        }
+    return angle.empty() ? 0.0 : *std::max_element(angle.begin(), angle.end());
+}
+
 }  // namespace ho2d

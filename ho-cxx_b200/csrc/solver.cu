@@ -98,6 +98,7 @@ Error Solver::setup() {
 Error Solver::setup_from_mesh() {
     setup_done_ = false;
     adj_.reset();
+    corner_ = largest_boundary_angle(mesh_) > kCornerAngle;
     HO2D_TRY(make_bases(in_.knod, mesh_.lnod, B_));
     make_metrics(mesh_, B_, M_);
     for (double j : M_.J)
@@ -709,7 +710,7 @@ Error Solver::poisson_solve() {
         const MfOp<double> A = make_op<double>(d, mesh_, K, false);
         const BicgVectors<double> v = krylov_vectors<double>(d, d.psi64.as<double>(), d.rhs.as<double>());
         int it = 0;
-        HO2D_TRY(run(A, v, d.pc64, solve_target(), it, d.graph64));
+        HO2D_TRY(run(A, v, d.pc64, fp64_target(), it, d.graph64));
         last_iters_ += it;
         const double bn = d.h_sc->bnorm2, rn = d.h_sc->rnorm2;
         finite = std::isfinite(bn) && std::isfinite(rn);

@@ -223,25 +223,33 @@ class Solver {
     // How far below the tolerance solves go. What the vertex coarse space's last iterates leave of
     // the residual sits in the few elements at a re-entrant corner, whose wall vorticity it
     // reaches undiluted, or where cells are stretched, and nearly none of it in the smooth modes;
-    // element constants left it evenly spread. The FP64 solve stops at a tenth of the tolerance;
-    // a refinement (of HO2D_MIXED_KRYLOV, and of every transposed solve) aims each sweep at a
-    // twentieth and accepts 0.3. None goes below 1e-13, where FP64 residuals round off. Errors of the
-    // vorticity at tolerance 1e-12 (2-norm and largest, against 1e-14): element constants stopped at the
-    // tolerance; the vertex space at 0.3 of it (FP64) or at it (refinement); as now.
-    //   backward-facing step (14,625 quads, K = 5), FP64     7.5e-11 4.5e-9, 1.4e-10 1.7e-8, 3.6e-11 4.4e-9
-    //   the same, HO2D_MIXED_KRYLOV                          2.8e-11 1.5e-9, 9.3e-11 1.3e-8, 7.8e-12 1.0e-9
-    //   channel O-grid (20 x 40, K = 3), FP64                3.9e-13 7.1e-12, 1.0e-12 1.5e-11, 2.5e-13 3.6e-12
-    //   the same, HO2D_MIXED_KRYLOV                          2.2e-13 4.1e-12, 8.9e-13 1.4e-11, 1.1e-13 1.9e-12
-    //   64 x 128 O-grid (K = 5), HO2D_MIXED_KRYLOV           9.3e-14 4.6e-12, 6.5e-13 2.2e-11, 9.5e-14 3.7e-12
-    // It costs about an iteration a solve. (A tenth in the refinement too costs another 4%, 0.15 in
-    // the FP64 solve saves 3% and leaves 8.0e-9 at the step's corner.) HO2D_MIXED's refinement stops
-    // at the tolerance, aiming at 0.3 of it: its FP32 stages leave 7e-9 on that step.
-    double solve_target() const { return std::min(tol_, std::max(0.1 * tol_, 1e-13)); }
+    // element constants left it evenly spread. So the FP64 solve stops at 0.3 of the tolerance, and
+    // at a tenth on a domain with a re-entrant corner; a refinement (of HO2D_MIXED_KRYLOV, and of every
+    // transposed solve) aims each sweep at a twentieth and accepts 0.3. None goes below 1e-13, where
+    // FP64 residuals round off. Errors of the vorticity at tolerance 1e-12 (2-norm and largest, against
+    // 1e-14): element constants stopped at the tolerance; the vertex space at 0.3 of it (FP64) or at it
+    // (refinement); as now.
+    //   step, 14,625 quads, K = 5, FP64       7.5e-11 4.5e-9,  1.4e-10 1.7e-8,  3.6e-11 4.4e-9
+    //   step, h = 1/24, K = 6, FP64           2.7e-10 1.9e-8,  2.6e-10 8.8e-8,  6.9e-11 2.3e-8
+    //   step, 14,625 quads, HO2D_MIXED_KRYLOV 2.8e-11 1.5e-9,  9.3e-11 1.3e-8,  7.8e-12 1.0e-9
+    //   channel 20 x 40, HO2D_MIXED_KRYLOV    2.2e-13 4.1e-12, 8.9e-13 1.4e-11, 1.1e-13 1.9e-12
+    //   O-grid 64 x 128, HO2D_MIXED_KRYLOV    9.3e-14 4.6e-12, 6.5e-13 2.2e-11, 9.5e-14 3.7e-12
+    // A margin costs about an iteration a solve: a tenth everywhere in FP64 would be 3% to 13% of a
+    // step, for errors that are below those of element constants already on cavities and large
+    // O-grids (256 x 512: 5.8e-11, 9.5e-12) and at 1e-12 on the channels (20 x 40: 3.9e-13, 1.0e-12). (A
+    // tenth in the refinement too costs another 4%; 0.15 at corners saves 3% and leaves 8.0e-9.)
+    // HO2D_MIXED's refinement stops at the tolerance, aiming at 0.3 of it: its FP32 stages leave 7e-9 on
+    // the step. The transposed FP64 solve stops at the tolerance without a corner: its errors are
+    // below those of element constants there.
+    bool corner_ = false;
+    double below(double margin) const { return std::min(tol_, std::max(margin * tol_, 1e-13)); }
+    double fp64_target() const { return below(corner_ ? 0.1 : 0.3); }
+    double transposed_target() const { return corner_ ? below(0.1) : tol_; }
     struct RefineGoal {
         double accept, aim;
     };
     RefineGoal refine_goal(bool fp64_stage) const {
-        const double accept = fp64_stage ? std::min(tol_, std::max(0.3 * tol_, 1e-13)) : tol_;
+        const double accept = fp64_stage ? below(0.3) : tol_;
         return {accept, fp64_stage ? std::min(0.3 * accept, std::max(0.05 * tol_, 3e-14)) : 0.3 * accept};
     }
     int max_iter_ = 500;

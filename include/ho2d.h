@@ -171,9 +171,10 @@ enum ho2d_setup_array {
 };
 int ho2d_get_poisson_setup(ho2d_solver* handle, int32_t which, int64_t len, double* buf);
 /* Poisson solve controls: relative tolerance on ||b - A psi|| / ||b|| (default 1e-12)
- * and iteration cap (default 500). Solves go below it (not below 1e-13), for the vorticity at
- * re-entrant corners: HO2D_FP64 and the adjoint in FP64 stop at a tenth of it, the refinement
- * of HO2D_MIXED_KRYLOV and of the adjoint in the mixed modes at 0.3. HO2D_MIXED stops at it. */
+ * and iteration cap (default 500). Solves go below it (not below 1e-13) where the vorticity
+ * needs it: HO2D_FP64 stops at 0.3 of it, on a domain with a re-entrant corner at a tenth; the
+ * refinement of HO2D_MIXED_KRYLOV, and of the adjoint in the mixed modes, at 0.3; the adjoint in
+ * FP64 at it, with a corner at a tenth; HO2D_MIXED at it. */
 int ho2d_set_poisson_tolerance(ho2d_solver* handle, double rel_tol, int32_t max_iter);
 /* Statistics of the last Poisson solve: Krylov iterations (inner iterations summed over
  * refinement sweeps) and final relative residual. */
