@@ -149,10 +149,10 @@ static __host__ __device__ constexpr unsigned rgrid_of(int N) {
 // everywhere: K = 6 on 256 x 512 elements 146 against 116.)
 template <int K, typename T>
 constexpr int kOperatorCtas = sizeof(T) == 4 ? 4 : (K <= 7 ? 3 : 1);
-// The residuals (k_mf_init, k_mf_residual): three in FP64 at orders 6 and 7 (init 66.1 and 61.2 us,
-// 70.3 and 68.9), elsewhere the compiler's own choice (0), which stops at 168 registers up to order
-// 5 and at 128 at order 2, where any stated minimum takes 160 (40.2 and 47.2 us), and does not
-// spill at order 8 (71.7 and 81.7).
+// The residuals (k_mf_init, k_mf_residual): three in FP64 at orders 6 and 7 (k_mf_init with two and with
+// three, the same meshes: 66.5 and 60.2 us, 71.0 and 67.3), elsewhere the compiler's own choice (0),
+// which stops at 168 registers up to order 5 and at 128 at order 2, where any stated minimum takes
+// 160 (500^2 elements: 42.3 us, 47.2 with it), and does not spill at order 8 (72.1, 81.7 with three).
 template <int K, typename T>
 constexpr int kResidualCtas = sizeof(T) == 8 && (K == 6 || K == 7) ? 3 : 0;
 
@@ -700,8 +700,10 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, kResidualCtas<K, T>) k_mf_re
 // programmatic primary (mf_apply_op): everything else is loaded while that kernel still runs,
 // and the traces (read through L2, since they are being written) after it has ended. A call
 // on 9,216 elements at K = 5 is bound by the two launches and the host's synchronisation.
-// Registers: the compiler's own choice (a minimum of three CTAs an SM: K = 2 on 500^2 elements 30.2
-// us, without it 22.7; K = 6 on 256^2 48.9 and 38.8; K = 8 on 200^2 62.8 and 47.9).
+// Registers: the compiler's own choice (K = 2 on 500^2 elements 28.0 us, with a minimum of three CTAs
+// an SM 30.2; K = 6 on 256^2 41.3 and 48.9; K = 8 on 200^2 53.1 and 62.8). With the traces before the
+// wait it would be 10 to 20% shorter by itself, but the call, whose two launches overlap, is 4 to
+// 13% shorter as it is (medians of 2,500 calls at 14 sizes, 12^2 elements to the fixed scratch's limit).
 template <int K, typename T>
 __global__ void __launch_bounds__(Rows<K>::THREADS)
     k_mf_apply(MfOp<T> op, const T* __restrict__ x, const T* xtv, const T* xtg, T* __restrict__ y) {
