@@ -701,9 +701,10 @@ __global__ void __launch_bounds__(Rows<K>::THREADS, kResidualCtas<K, T>) k_mf_re
 // and the traces (read through L2, since they are being written) after it has ended. A call
 // on 9,216 elements at K = 5 is bound by the two launches and the host's synchronisation.
 // Registers: the compiler's own choice (K = 2 on 500^2 elements 28.0 us, with a minimum of three CTAs
-// an SM 30.2; K = 6 on 256^2 41.3 and 48.9; K = 8 on 200^2 53.1 and 62.8). With the traces before the
-// wait it would be 10 to 20% shorter by itself, but the call, whose two launches overlap, is 4 to
-// 13% shorter as it is (medians of 2,500 calls at 14 sizes, 12^2 elements to the fixed scratch's limit).
+// an SM 30.2; K = 6 on 256^2 41.3 and 48.9; K = 8 on 200^2 53.1 and 62.8). Without the wait, all loads
+// together, it took 22.7, 38.8 and 47.9 us by itself, but the call, whose two launches overlap, is 4
+// to 13% shorter as it is (medians of 2,500 calls at 14 sizes, 12^2 elements to the fixed scratch's
+// limit).
 template <int K, typename T>
 __global__ void __launch_bounds__(Rows<K>::THREADS)
     k_mf_apply(MfOp<T> op, const T* __restrict__ x, const T* xtv, const T* xtg, T* __restrict__ y) {
